@@ -1382,9 +1382,9 @@ int bf_probabilities(bf_state* hst, const int32_t* qubits, const int8_t* values,
   return guarded([&]() {
     if (!st || !out) fail(BF_EINVAL, "null argument");
     DeviceGuard dg(st->device);
-    std::vector<double> p;
-    marginal_probs(*st, qubits, values, nq, p);
-    std::memcpy(out, p.data(), p.size() * sizeof(double));
+    uint64_t count = 0;
+    const double* p = marginal_probs(*st, qubits, values, nq, &count);
+    std::memcpy(out, p, count * sizeof(double));
   });
 }
 

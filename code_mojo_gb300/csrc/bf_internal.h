@@ -269,7 +269,7 @@ struct State {
   // reduction partials
   double* d_partial = nullptr;
   double* h_partial = nullptr;
-  size_t partial_cap = 0;
+  size_t partial_cap = 0, h_partial_cap = 0;  // in pairs of doubles
   // error flag of kernels with bounded waits (device word, pinned copy)
   int* d_flag = nullptr;
   int* h_flag = nullptr;
@@ -355,8 +355,9 @@ void inner_product(State& a, State& b, double* re, double* im);
 // complex64: restore the norm measured by launch_norm_before (or 1), stream-ordered
 void launch_norm_before(State& st);
 void launch_renormalize(State& st, bool unit_before);
-void ensure_partials(State& st, size_t blocks);  // 2*blocks doubles, device + pinned host
-void marginal_probs(State& st, const int32_t* q, const int8_t* values, int32_t nq, std::vector<double>& out);
+// at least 2*blocks doubles on the device and 2*host_blocks pinned
+void ensure_partials(State& st, size_t blocks, size_t host_blocks);
+const double* marginal_probs(State& st, const int32_t* q, const int8_t* values, int32_t nq, uint64_t* count);
 void measure(State& st, const int32_t* q, const int8_t* values, int32_t nq, int64_t seed, uint64_t* outcome,
              double* prob);
 void probs_topk(State& st, int k, uint64_t* idx, double* probs);

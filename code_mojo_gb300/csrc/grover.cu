@@ -284,7 +284,7 @@ static void diffuser_p(State& st, DiffArgs& a) {
   if (slots > 0x7fffffffull) fail(BF_EUNSUPPORTED, "too many diffuser blocks");
   // partials (float4 per slot) then 2*mean (float4 per block), in the partials buffer
   size_t need = (size_t)(slots + a.blocks) * sizeof(float4);
-  ensure_partials(st, (need + 2 * sizeof(double) - 1) / (2 * sizeof(double)));
+  ensure_partials(st, (need + 2 * sizeof(double) - 1) / (2 * sizeof(double)), 0);
   float4* partial = reinterpret_cast<float4*>(st.d_partial);
   float4* mean2 = partial + slots;
   auto* s = static_cast<typename P::Glob*>(st.amp);
@@ -658,7 +658,7 @@ void launch_grover_loop(State& st, const uint64_t* marked, int nmarked, int iter
   G = (st.N + a.chunk - 1) / a.chunk;
   // partial sums (2 x G float4), the arrival counter after them
   size_t bytes = 2 * G * sizeof(float4) + 16;
-  ensure_partials(st, (bytes + 2 * sizeof(double) - 1) / (2 * sizeof(double)));
+  ensure_partials(st, (bytes + 2 * sizeof(double) - 1) / (2 * sizeof(double)), 0);
   a.partial = reinterpret_cast<float4*>(st.d_partial);
   a.bar = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(st.d_partial) + 2 * G * sizeof(float4));
   a.flag = state_flag(st);

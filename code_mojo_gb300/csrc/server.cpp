@@ -156,7 +156,7 @@ static void worker_main(Server* sv, int slot) {
     st.stream = s_hi;
     // size the work buffers for the typical request up front
     upload_program_reserve(st, 16384);
-    ensure_partials(st, 1 << 15);
+    ensure_partials(st, 1 << 15, 1 << 15);
     BF_CUDA(cudaStreamSynchronize(st.stream));
   } catch (const Error&) {
     ready = false;

@@ -125,22 +125,28 @@ __global__ void __launch_bounds__(256) k_norm2(const T* __restrict__ s, uint64_t
   }
 }
 
-void ensure_partials(State& st, size_t blocks) {
-  if (st.partial_cap >= blocks) return;
-  blocks = std::max(blocks, 2 * st.partial_cap);
-  dev_free(st, st.d_partial);
-  host_retire(st, st.h_partial);
-  st.d_partial = nullptr;
-  st.h_partial = nullptr;
-  st.partial_cap = 0;
-  st.d_partial = static_cast<double*>(dev_alloc(st, 2 * blocks * sizeof(double)));
-  st.h_partial = static_cast<double*>(host_alloc(2 * blocks * sizeof(double)));
-  st.partial_cap = blocks;
+void ensure_partials(State& st, size_t blocks, size_t host_blocks) {
+  if (st.partial_cap < blocks) {
+    blocks = std::max(blocks, 2 * st.partial_cap);
+    dev_free(st, st.d_partial);
+    st.d_partial = nullptr;
+    st.partial_cap = 0;
+    st.d_partial = static_cast<double*>(dev_alloc(st, 2 * blocks * sizeof(double)));
+    st.partial_cap = blocks;
+  }
+  if (st.h_partial_cap < host_blocks) {
+    host_blocks = std::max(host_blocks, 2 * st.h_partial_cap);
+    host_retire(st, st.h_partial);
+    st.h_partial = nullptr;
+    st.h_partial_cap = 0;
+    st.h_partial = static_cast<double*>(host_alloc(2 * host_blocks * sizeof(double)));
+    st.h_partial_cap = host_blocks;
+  }
 }
 
 double reduce_norm2(State& st) {
   unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((st.N + 255) / 256, (uint64_t)st.num_sms * 8));
-  ensure_partials(st, blocks);
+  ensure_partials(st, blocks, blocks);
   if (st.dtype == BF_C128)
     k_norm2<double2><<<blocks, 256, 0, st.stream>>>(static_cast<const double2*>(st.amp), st.N, st.d_partial);
   else
@@ -218,7 +224,7 @@ __global__ void __launch_bounds__(256) k_inner(const TA* __restrict__ a, const T
 void inner_product(State& a, State& b, double* re, double* im) {
   if (a.n != b.n) fail(BF_EINVAL, "inner product of states with %d and %d qubits", a.n, b.n);
   unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.N + 255) / 256, (uint64_t)a.num_sms * 8));
-  ensure_partials(a, 2 * (size_t)blocks);
+  ensure_partials(a, 2 * (size_t)blocks, 2 * (size_t)blocks);
   // b's pending work must finish before a's stream reads it
   cudaEvent_t ev;
   BF_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));

@@ -1077,7 +1077,7 @@ __global__ void k_digit_scale(const double* __restrict__ partial, int blocks, in
 
 void launch_digit_scale(State& st, int* d_exp) {
   const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((st.N + 255) / 256, (uint64_t)st.num_sms * 8));
-  ensure_partials(st, blocks);
+  ensure_partials(st, blocks, 0);
   launch_norm2_partials(st, blocks);
   k_digit_scale<<<1, 32, 0, st.stream>>>(st.d_partial, (int)blocks, d_exp);
   BF_CUDA(cudaGetLastError());
