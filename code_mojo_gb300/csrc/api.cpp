@@ -326,11 +326,6 @@ static void fused_pair_matrix(const bf_op& t0, const bf_op& t1, int& q_low, std:
     }
 }
 
-// Grover loops run for states of up to kLoopAlwaysQubits qubits, and for
-// larger ones only when grover_loop_large (a server slot keeps long searches
-// as short per-op kernels so that other requests get SMs between them).
-constexpr int kLoopAlwaysQubits = 22;
-
 // Tensor cores or CUDA cores for one 12-qubit pass: the CUDA-core tile
 // kernel's work in units of one dense gate over the tile, against the blocks
 // the pass needs (one block costs about kBlockUnits dense gates: measured on
@@ -403,8 +398,7 @@ static bool norm_preserving(const bf_op* ops, int64_t nops) {
 // tensor: tile passes as tensor-core block passes (12-qubit tiles), in
 // `format` (BLOCK_TF32 for complex64, BLOCK_DIGITS for complex128)
 static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opts& o, std::vector<Step>& steps,
-                        Program& pg, bool grover_loop_large = true, bool tensor = false,
-                        BlockFormat format = BLOCK_TF32) {
+                        Program& pg, bool tensor = false, BlockFormat format = BLOCK_TF32) {
   std::vector<TileOp>& prog = pg.ops;
   const bool fused = o.strategy == BF_STRATEGY_GPU_FUSED;
   tensor = tensor && fused && n >= kBlockTileQubits;
@@ -626,8 +620,8 @@ static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opt
       case BF_OP_CLASSICAL_ORACLE: {  // classical_oracle (grover.mojo:64-66)
         flush();
         int64_t reps = grover_loop_reps(n, ops, nops, i);
-        if (reps >= 2 && (grover_loop_large || n <= kLoopAlwaysQubits)) {
-          // repeated (oracle, full diffuser) iterations: one cooperative loop
+        if (reps >= 2) {
+          // repeated (oracle, full diffuser) iterations: one affine map of the state
           std::vector<uint64_t> idx;
           for (int64_t k = 0; k < op.nqubits; ++k) idx.push_back((uint64_t)op.data[k]);
           std::sort(idx.begin(), idx.end());
@@ -781,8 +775,8 @@ static void plan_key(std::vector<unsigned char>& k, const State& st, const bf_op
     const unsigned char* c = static_cast<const unsigned char*>(p);
     k.insert(k.end(), c, c + n);
   };
-  const int32_t head[8] = {st.n, st.dtype, (int32_t)format, st.shared_gpu ? 1 : 0, o.strategy, o.tile_qubits,
-                           (int32_t)o.specialized, o.tensor_blocks};
+  const int32_t head[7] = {st.n, st.dtype, (int32_t)format, o.strategy, o.tile_qubits, (int32_t)o.specialized,
+                           o.tensor_blocks};
   k.reserve(sizeof head + (size_t)nops * sizeof(bf_op));
   put(head, sizeof head);
   for (int64_t i = 0; i < nops; ++i) {
@@ -818,7 +812,7 @@ void execute_ops(State& st, const bf_op* ops, int64_t nops, bf_exec_opts o) {
     }
   if (hit == entries.size()) {
     PlanCache::Entry ne;
-    build_steps(st.n, ops, nops, o, ne.steps, ne.prog, !st.shared_gpu, o.tensor_blocks != 0, format);
+    build_steps(st.n, ops, nops, o, ne.steps, ne.prog, o.tensor_blocks != 0, format);
     ne.key = std::move(key);
     ne.id = st.plans->next_id++;
     entries.insert(entries.begin(), std::move(ne));
@@ -1555,7 +1549,7 @@ int bf_plan_stats(int32_t n, const bf_op* ops, int64_t nops, const bf_exec_opts*
     if (o.validate) validate_ops(n, ops, nops);
     std::vector<Step> steps;
     Program prog;
-    build_steps(n, ops, nops, o, steps, prog, true, o.tensor_blocks != 0,
+    build_steps(n, ops, nops, o, steps, prog, o.tensor_blocks != 0,
                 o.plan_dtype == BF_C64 ? BLOCK_TF32 : BLOCK_DIGITS);
     int64_t t = 0, g = 0, x = 0, bp = 0, nb = 0;
     double bytes = 0;
@@ -1572,7 +1566,7 @@ int bf_plan_stats(int32_t n, const bf_op* ops, int64_t nops, const bf_exec_opts*
         bytes += gate_bytes_fraction(s.gate);
       } else if (s.kind == Step::GROVER_LOOP) {
         ++x;
-        bytes += 2.0 * (s.reps + 1);
+        bytes += 3.0;  // read for the sum, read and written by the update
       } else {
         ++x;
         bytes += (s.kind == Step::SWAPBITS) ? 1.0

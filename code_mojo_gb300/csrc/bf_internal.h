@@ -275,7 +275,7 @@ struct State {
   int* h_flag = nullptr;
   bool flag_used = false;
   // the state runs in a server slot that shares the GPU with other slots:
-  // long persistent kernels (grid-wide Grover loops) are not used
+  // kernels whose CTAs wait for one another (Grover loops) stay narrow
   bool shared_gpu = false;
   // block descriptors and matrix images of tensor-core passes (device) and
   // their pinned staging; uploaded with the tile program
@@ -364,7 +364,7 @@ void probs_topk(State& st, int k, uint64_t* idx, double* probs);
 void launch_grover_inversion0(State& st, const int32_t* q, int32_t nq);
 void launch_grover_diffuser(State& st, const int32_t* q, int32_t nq);
 void launch_classical_oracle(State& st, const double* idx, int64_t count);
-// iters x (negate marked[0..nmarked), diffuser over every qubit) in one launch
+// iters x (negate marked[0..nmarked), diffuser over every qubit) as one affine map, in one launch
 void launch_grover_loop(State& st, const uint64_t* marked, int nmarked, int iters);
 int grover_loop_max_marked();
 // sum |amp|^2 of caller memory with the library's static scratch (noalloc.cu)

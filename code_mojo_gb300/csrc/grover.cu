@@ -11,6 +11,7 @@
 // (grover_classical.mojo:318); this pass uses 2 * mean - x for both parts,
 // the inversion about the mean for complex amplitudes.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -310,25 +311,36 @@ void launch_grover_diffuser(State& st, const int32_t* q, int32_t nq) {
 // ---- Grover search loop ------------------------------------------------------
 // `iters` repetitions of (classical oracle, diffuser over every qubit) -- the
 // body of grover_search with the classical replacements (grover.mojo:64-94,
-// grover_classical.mojo:284-326) -- in one cooperative launch.  Each CTA owns
-// a fixed contiguous chunk of the state.  Pass p (0..iters) reads the chunk,
-// applies the diffuser update of iteration p-1 (x <- 2*mean - x, the mean
-// coming from the partial sums of pass p-1), then the oracle of iteration p
-// (negate the marked amplitudes) and sums the result for the next mean; one
-// grid barrier separates the passes.  Per iteration this is one read and one
-// write of the state and no launch, against three launches and 1.5 passes for
-// the per-op form.  The partial sums alternate between two buffers, so a CTA
-// that runs ahead into pass p+1 never overwrites sums another CTA is still
-// reading in pass p.
+// grover_classical.mojo:284-326) -- in one launch and one read-modify-write of
+// the state, whatever the iteration count.
+//
+// With k marked amplitudes (sum W) and the N - k others (sum U), an iteration
+// adds m = 2 (U - W) / N to every marked amplitude and maps every other one
+// to m - x.  In the coordinates u = U / sqrt(N - k), w = W / sqrt(k) that is a
+// rotation by 2 theta, sin(theta) = sqrt(k / N) (the two-dimensional picture
+// of the search), so r iterations are the rotation by phi = 2 r theta, and
+//   x -> (-1)^r x + c   (unmarked),  c = (U_r - (-1)^r U_0) / (N - k)
+//   x -> x + d          (marked),    d = (W_r - W_0) / k
+// with c and d linear in U_0 and W_0.  The host forms the four coefficients
+// (grover_coefficients); the kernel sums the state, meets at one grid barrier
+// and adds c or d.
+//
+// Bound by memory: one read for the sum, one read and one write for the
+// update (3S; the sum's second read comes from L2 up to about 2^22
+// amplitudes).  At 20 qubits, complex128, 804 iterations: 10.7 ms with a
+// sweep and a grid barrier per iteration, 0.024 ms like this.  x is rounded
+// once instead of once per iteration: served searches of 10 to 20 qubits went
+// from 5.5e-13 to 2.6e-14 off the 64-bit probabilities.
 struct LoopArgs {
   uint64_t N;
   uint64_t chunk;         // amplitudes per CTA
-  int32_t iters;
   int32_t nmarked;        // indices negated by the oracle (odd multiplicity)
   uint64_t marked[8];
-  int32_t n;              // qubits: 2 * mean = sum * 2^(1-n)
+  int32_t odd;            // 1: an odd number of iterations (the sign of x)
+  double cu, cw;          // c = cu U_0 + cw W_0
+  double du, dw;          // d = du U_0 + dw W_0
   uint32_t spin_limit;    // polls of 64 ns before a barrier wait gives up
-  float4* partial;        // 2 x gridDim.x
+  float4* partial;        // gridDim.x
   unsigned int* bar;      // arrival counter, zero at launch
   int* flag;              // set to 1 when a barrier wait expires
 };
@@ -383,286 +395,150 @@ __device__ __forceinline__ void block_sum2(dfl& r, dfl& im, dfl* wr, dfl* wi) {
   }
 }
 
-template <class P>
-__device__ __forceinline__ void loop_update(typename P::R& x, const float4 m) {
-  if constexpr (std::is_same<P, PolDF>::value) {
-    x.re = df_sub(dfl{m.x, m.y}, x.re);
-    x.im = df_sub(dfl{m.z, m.w}, x.im);
-  } else if constexpr (std::is_same<P, PolF32>::value) {
-    x.re = (m.x + m.y) - x.re;
-    x.im = (m.z + m.w) - x.im;
-  } else {
-    x.re = ((double)m.x + (double)m.y) - x.re;
-    x.im = ((double)m.z + (double)m.w) - x.im;
-  }
+// sign * x + c: complex128 in FP64 (two DADD per amplitude stay under the
+// pass's HBM time), complex64 with c as an FP32 pair
+__device__ __forceinline__ double2 loop_shift(double2 x, bool neg, double cr, double ci) {
+  return make_double2((neg ? -x.x : x.x) + cr, (neg ? -x.y : x.y) + ci);
+}
+__device__ __forceinline__ float2 loop_shift(float2 x, bool neg, float2 cr, float2 ci) {
+  return make_float2((cr.x + (neg ? -x.x : x.x)) + cr.y, (ci.x + (neg ? -x.y : x.y)) + ci.y);
+}
+__device__ __forceinline__ float2 loop_pair(double v) {
+  const float hi = (float)v;
+  return make_float2(hi, (float)(v - (double)hi));
 }
 
-template <class P>
-__device__ __forceinline__ void loop_accumulate(const typename P::R& x, dfl& sr, dfl& si) {
-  if constexpr (std::is_same<P, PolDF>::value) {
-    sr = df_add(sr, x.re);
-    si = df_add(si, x.im);
-  } else if constexpr (std::is_same<P, PolF32>::value) {
-    sr = df_add(sr, dfl{x.re, 0.f});
-    si = df_add(si, dfl{x.im, 0.f});
-  } else {
-    sr = df_add(sr, df_from_double(x.re));
-    si = df_add(si, df_from_double(x.im));
-  }
-}
-
-template <class P>
-__device__ __forceinline__ void loop_negate(typename P::R& x) {
-  if constexpr (std::is_same<P, PolDF>::value) {
-    x.re = df_neg(x.re);
-    x.im = df_neg(x.im);
-  } else {
-    x.re = -x.re;
-    x.im = -x.im;
-  }
-}
-
-template <class P>
-__global__ void __launch_bounds__(256) k_grover_loop(typename P::Glob* __restrict__ s, LoopArgs a) {
+template <class T>
+__global__ void __launch_bounds__(256) k_grover_loop(T* __restrict__ s, LoopArgs a) {
   __shared__ dfl wr[8], wi[8];
-  __shared__ float4 m2_sh;
+  __shared__ double shift[4];  // c (re, im), d (re, im)
+  __shared__ double2 mk[8];    // the marked amplitudes before the loop
   const uint64_t begin = (uint64_t)blockIdx.x * a.chunk;
   const uint64_t end = min(begin + a.chunk, a.N);
   const unsigned int G = gridDim.x;
-  const float sc = ldexpf(1.0f, 1 - a.n);
-  for (int p = 0; p <= a.iters; ++p) {
-    float4 m2 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p > 0) {
-      const float4* part = a.partial + (size_t)((p - 1) & 1) * G;
-      dfl r{0.f, 0.f}, im{0.f, 0.f};
-      for (unsigned int c = threadIdx.x; c < G; c += blockDim.x) {
-        float4 q = __ldcg(part + c);
-        r = df_add(r, dfl{q.x, q.y});
-        im = df_add(im, dfl{q.z, q.w});
-      }
-      block_sum2(r, im, wr, wi);
-      if (threadIdx.x == 0) m2_sh = make_float4(r.hi * sc, r.lo * sc, im.hi * sc, im.lo * sc);
-      __syncthreads();
-      m2 = m2_sh;
+  // every CTA reads the marked amplitudes before any CTA writes the state
+  if ((int)threadIdx.x < a.nmarked) {
+    const T v = s[a.marked[threadIdx.x]];
+    mk[threadIdx.x] = make_double2((double)v.x, (double)v.y);
+  }
+  // eight loads in flight per thread before any use
+  constexpr int kU = 8;
+  dfl sr{0.f, 0.f}, si{0.f, 0.f};
+  for (uint64_t base = begin + threadIdx.x; base < end; base += kU * blockDim.x) {
+    T v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t i = base + (uint64_t)u * blockDim.x;
+      v[u] = i < end ? s[i] : T{};
     }
-    const bool last = p == a.iters;
-    dfl sr{0.f, 0.f}, si{0.f, 0.f};
-    // eight loads in flight per thread before any use
-    constexpr int kU = 8;
-    for (uint64_t base = begin + threadIdx.x; base < end; base += kU * blockDim.x) {
-      typename P::Glob v[kU];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const uint64_t i = base + (uint64_t)u * blockDim.x;
-        if (i < end) v[u] = s[i];
-      }
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const uint64_t i = base + (uint64_t)u * blockDim.x;
-        if (i >= end) break;
-        typename P::R x = P::from_glob(v[u]);
-        if (p > 0) loop_update<P>(x, m2);
-        if (!last) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (k < a.nmarked && i == a.marked[k]) loop_negate<P>(x);
-          loop_accumulate<P>(x, sr, si);
-        }
-        s[i] = P::to_glob(x);
-      }
-    }
-    if (last) break;
-    __syncthreads();  // wr/wi reuse
-    block_sum2(sr, si, wr, wi);
-    if (threadIdx.x == 0) a.partial[(size_t)(p & 1) * G + blockIdx.x] = make_float4(sr.hi, sr.lo, si.hi, si.lo);
-    if (G > 1) {
-      if (!loop_barrier(a, (unsigned int)(p + 1) * G)) return;
-    } else {
-      __syncthreads();
+    for (int u = 0; u < kU; ++u) {
+      dfl xr, xi;
+      amp_df<T>(v[u], xr, xi);
+      sr = df_add(sr, xr);
+      si = df_add(si, xi);
     }
   }
-}
-
-// Cluster form, for states that fit in the shared memory of one thread-block
-// cluster (up to 16 CTAs of 128 KiB): each CTA keeps its chunk in shared
-// memory for all iterations, the partial sums travel through distributed
-// shared memory and the hardware cluster barrier separates the passes -- no
-// global traffic between the first load and the last store, and no waits of
-// our own.
-constexpr int kClusterThreads = 512;
-constexpr uint32_t kClusterChunkBytes = 128 * 1024;
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile(
-      "barrier.cluster.arrive.release.aligned;\n\t"
-      "barrier.cluster.wait.acquire.aligned;" ::
-          : "memory");
-}
-
-__device__ __forceinline__ float4 ld_cluster_f4(const float4* local, uint32_t rank) {
-  uint32_t la = (uint32_t)__cvta_generic_to_shared(local), ra;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(la), "r"(rank));
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(ra)
-               : "memory");
-  return v;
-}
-
-template <class P>
-__global__ void __launch_bounds__(kClusterThreads) k_grover_cluster(typename P::Glob* __restrict__ s, LoopArgs a,
-                                                                      uint32_t csize) {
-  using S = typename P::Smem;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  S* amp = reinterpret_cast<S*>(smem_raw);
-  __shared__ float4 part[2];  // this CTA's partial sums, by pass parity
-  __shared__ dfl wr[kClusterThreads / 32], wi[kClusterThreads / 32];
-  __shared__ float4 m2_sh;
-  const uint32_t rank = cluster_rank();
-  const int cnt = (int)a.chunk;
-  const uint64_t begin = (uint64_t)rank * a.chunk;
-  for (int e = threadIdx.x; e < cnt; e += kClusterThreads) amp[e] = P::to_smem(P::from_glob(s[begin + e]));
-  __syncthreads();
-  const float sc = ldexpf(1.0f, 1 - a.n);
-  for (int p = 0; p <= a.iters; ++p) {
-    float4 m2 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p > 0) {
-      if (threadIdx.x < 32) {  // every CTA sums the cluster's partials in the same order
-        dfl r{0.f, 0.f}, im{0.f, 0.f};
-        if (threadIdx.x < csize) {
-          const float4 q = ld_cluster_f4(&part[(p - 1) & 1], threadIdx.x);
-          r = dfl{q.x, q.y};
-          im = dfl{q.z, q.w};
-        }
-        for (int off = 16; off > 0; off >>= 1) {
-          r = df_add(r, dfl{__shfl_down_sync(0xffffffffu, r.hi, off), __shfl_down_sync(0xffffffffu, r.lo, off)});
-          im = df_add(im, dfl{__shfl_down_sync(0xffffffffu, im.hi, off), __shfl_down_sync(0xffffffffu, im.lo, off)});
-        }
-        if (threadIdx.x == 0) m2_sh = make_float4(r.hi * sc, r.lo * sc, im.hi * sc, im.lo * sc);
-      }
-      __syncthreads();
-      m2 = m2_sh;
+  block_sum2(sr, si, wr, wi);
+  if (threadIdx.x == 0) a.partial[blockIdx.x] = make_float4(sr.hi, sr.lo, si.hi, si.lo);
+  if (G > 1) {
+    if (!loop_barrier(a, G)) return;
+  } else {
+    __syncthreads();
+  }
+  sr = si = dfl{0.f, 0.f};
+  for (unsigned int c = threadIdx.x; c < G; c += blockDim.x) {
+    const float4 q = __ldcg(a.partial + c);
+    sr = df_add(sr, dfl{q.x, q.y});
+    si = df_add(si, dfl{q.z, q.w});
+  }
+  block_sum2(sr, si, wr, wi);
+  if (threadIdx.x == 0) {
+    double w0 = 0, w1 = 0;
+    for (int k = 0; k < a.nmarked; ++k) {
+      w0 += mk[k].x;
+      w1 += mk[k].y;
     }
-    const bool last = p == a.iters;
-    dfl sr{0.f, 0.f}, si{0.f, 0.f};
-    for (int e = threadIdx.x; e < cnt; e += kClusterThreads) {
-      typename P::R x = P::from_smem(amp[e]);
-      if (p > 0) loop_update<P>(x, m2);
-      if (!last) {
-        const uint64_t i = begin + (uint64_t)e;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (k < a.nmarked && i == a.marked[k]) loop_negate<P>(x);
-        loop_accumulate<P>(x, sr, si);
-      }
-      amp[e] = P::to_smem(x);
-    }
-    if (last) break;
-    block_sum2(sr, si, wr, wi);
-    if (threadIdx.x == 0) part[p & 1] = make_float4(sr.hi, sr.lo, si.hi, si.lo);
-    cluster_sync_all();
+    const double u0 = ((double)sr.hi + (double)sr.lo) - w0, u1 = ((double)si.hi + (double)si.lo) - w1;
+    shift[0] = a.cu * u0 + a.cw * w0;
+    shift[1] = a.cu * u1 + a.cw * w1;
+    shift[2] = a.du * u0 + a.dw * w0;
+    shift[3] = a.du * u1 + a.dw * w1;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < cnt; e += kClusterThreads) s[begin + e] = P::to_glob(P::from_smem(amp[e]));
-  // the other CTAs may still be reading this CTA's partials
-  cluster_sync_all();
-}
-
-// launches the cluster form when the state fits; false otherwise
-template <class P>
-static bool try_grover_cluster(State& st, LoopArgs& a) {
-  const uint64_t cap = kClusterChunkBytes / sizeof(typename P::Smem);
-  uint32_t C = 1;
-  while ((uint64_t)C * cap < st.N) C <<= 1;
-  if (C > 16) return false;
-  a.chunk = st.N / C;
-  const size_t smem = (size_t)a.chunk * sizeof(typename P::Smem);
-  static PerDeviceOnce configured;  // one per instantiation of P
-  configured.run(st.device, [] {
-    BF_CUDA(cudaFuncSetAttribute(k_grover_cluster<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kClusterChunkBytes));
-    BF_CUDA(cudaFuncSetAttribute(k_grover_cluster<P>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  });
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(C);
-  cfg.blockDim = dim3(kClusterThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st.stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, k_grover_cluster<P>, &cfg) != cudaSuccess || clusters < 1) {
-    cudaGetLastError();
-    return false;
+  const bool neg = a.odd != 0;
+  auto as_shift = [](double v) {
+    if constexpr (sizeof(T) == 16) return v;
+    else return loop_pair(v);
+  };
+  const auto cr = as_shift(shift[0]), ci = as_shift(shift[1]);
+  for (uint64_t base = begin + threadIdx.x; base < end; base += kU * blockDim.x) {
+    T v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t i = base + (uint64_t)u * blockDim.x;
+      if (i < end) v[u] = s[i];
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t i = base + (uint64_t)u * blockDim.x;
+      if (i < end) s[i] = loop_shift(v[u], neg, cr, ci);
+    }
   }
-  BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_cluster<P>, static_cast<typename P::Glob*>(st.amp), a, C));
-  st.launches++;
-  return true;
+  // the CTA's own marked amplitudes, once its unmarked update is done
+  __syncthreads();
+  if ((int)threadIdx.x < a.nmarked) {
+    const uint64_t i = a.marked[threadIdx.x];
+    if (i >= begin && i < end) {
+      const double2 x = mk[threadIdx.x];
+      T v;
+      v.x = (decltype(v.x))(x.x + shift[2]);
+      v.y = (decltype(v.y))(x.y + shift[3]);
+      s[i] = v;
+    }
+  }
 }
 
 int grover_loop_max_marked() { return 8; }
 
-void launch_grover_loop(State& st, const uint64_t* marked, int nmarked, int iters) {
-  if (iters <= 0) return;
-  if (nmarked < 0 || nmarked > 8) fail(BF_EINVAL, "internal: %d oracle indices in a Grover loop", nmarked);
-  LoopArgs a;
-  std::memset(&a, 0, sizeof a);
-  a.N = st.N;
-  a.n = st.n;
-  a.iters = iters;
-  a.nmarked = nmarked;
-  for (int k = 0; k < nmarked; ++k) a.marked[k] = marked[k];
-  switch (st.prec) {
-    case PREC_F64:
-      if (try_grover_cluster<PolF64>(st, a)) return;
-      break;
-    case PREC_DF:
-      if (try_grover_cluster<PolDF>(st, a)) return;
-      break;
-    default:
-      if (try_grover_cluster<PolF32>(st, a)) return;
-      break;
-  }
-  a.spin_limit = 1u << 25;  // x 64 ns sleeps: about 2 s
-  // chunks of at least 4096 amplitudes
+// The coefficients of c and d (above).  Differences of nearly equal terms are
+// taken as products of half-angle sines and cosines, so each coefficient is
+// good to about phi 2^-53 relative to the larger of its two terms.
+static void grover_coefficients(LoopArgs& a, int iters) {
+  const double N = (double)a.N, k = (double)a.nmarked, rest = N - k;
+  const double phi = 2.0 * iters * std::asin(std::sqrt(k / N));
+  const double half_s = std::sin(0.5 * phi), half_c = std::cos(0.5 * phi), sn = std::sin(phi);
+  a.odd = iters & 1;
+  // cos(phi) - (-1)^r and cos(phi) - 1
+  const double cos_sign = a.odd ? 2.0 * half_c * half_c : -2.0 * half_s * half_s;
+  const double cos_one = -2.0 * half_s * half_s;
+  const bool both = k > 0 && rest > 0;
+  a.cu = rest > 0 ? cos_sign / rest : 0.0;
+  a.cw = both ? -sn / std::sqrt(rest * k) : 0.0;
+  a.du = both ? sn / std::sqrt(rest * k) : 0.0;
+  a.dw = k > 0 ? cos_one / k : 0.0;
+}
+
+template <class T>
+static void launch_grover_t(State& st, LoopArgs& a) {
   int per_sm = 0;
-  const void* fn = nullptr;
-  switch (st.prec) {
-    case PREC_F64: fn = (const void*)k_grover_loop<PolF64>; break;
-    case PREC_DF: fn = (const void*)k_grover_loop<PolDF>; break;
-    default: fn = (const void*)k_grover_loop<PolF32>; break;
-  }
-  BF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
-  uint64_t resident = (uint64_t)std::max(1, per_sm) * (uint64_t)st.num_sms;
-  // a server slot shares the GPU: its loop holds at most kSharedLoopCtas
-  // SMs' worth of CTAs for the whole search, so the other slots keep the rest
-  // (per-op kernels instead would issue four launches per iteration from
-  // every slot at once)
+  BF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_grover_loop<T>, 256, 0));
+  const uint64_t resident = (uint64_t)std::max(1, per_sm) * (uint64_t)st.num_sms;
+  // a server slot shares the GPU: its CTAs wait for one another at the
+  // barrier, so it takes at most kSharedLoopCtas and the other slots keep the rest
   constexpr uint64_t kSharedLoopCtas = 16;
   const uint64_t cap = st.shared_gpu ? kSharedLoopCtas : (uint64_t)2 * st.num_sms;
+  // chunks of at least 4096 amplitudes
   uint64_t G = std::max<uint64_t>(1, std::min<uint64_t>(std::min(cap, resident), st.N >> 12));
   a.chunk = (st.N + G - 1) / G;
   a.chunk = (a.chunk + 255) & ~255ull;
   G = (st.N + a.chunk - 1) / a.chunk;
-  // partial sums (2 x G float4), the arrival counter after them
-  size_t bytes = 2 * G * sizeof(float4) + 16;
+  // partial sums (G float4), the arrival counter after them
+  const size_t bytes = G * sizeof(float4) + 16;
   ensure_partials(st, (bytes + 2 * sizeof(double) - 1) / (2 * sizeof(double)), 0);
   a.partial = reinterpret_cast<float4*>(st.d_partial);
-  a.bar = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(st.d_partial) + 2 * G * sizeof(float4));
+  a.bar = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(st.d_partial) + G * sizeof(float4));
   a.flag = state_flag(st);
-  BF_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), st.stream));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)G);
   cfg.blockDim = dim3(256);
@@ -671,14 +547,27 @@ void launch_grover_loop(State& st, const uint64_t* marked, int nmarked, int iter
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  switch (st.prec) {
-    case PREC_F64: BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_loop<PolF64>, static_cast<double2*>(st.amp), a)); break;
-    case PREC_DF: BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_loop<PolDF>, static_cast<double2*>(st.amp), a)); break;
-    default: BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_loop<PolF32>, static_cast<float2*>(st.amp), a)); break;
+  if (G > 1) {
+    BF_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), st.stream));
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
   }
+  BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_loop<T>, static_cast<T*>(st.amp), a));
   st.launches++;
+}
+
+void launch_grover_loop(State& st, const uint64_t* marked, int nmarked, int iters) {
+  if (iters <= 0) return;
+  if (nmarked < 0 || nmarked > 8) fail(BF_EINVAL, "internal: %d oracle indices in a Grover loop", nmarked);
+  LoopArgs a;
+  std::memset(&a, 0, sizeof a);
+  a.N = st.N;
+  a.nmarked = nmarked;
+  for (int k = 0; k < nmarked; ++k) a.marked[k] = marked[k];
+  grover_coefficients(a, iters);
+  a.spin_limit = 1u << 25;  // x 64 ns sleeps: about 2 s
+  if (st.dtype == BF_C128) launch_grover_t<double2>(st, a);
+  else launch_grover_t<float2>(st, a);
 }
 
 }  // namespace bf

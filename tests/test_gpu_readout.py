@@ -1,9 +1,11 @@
-"""Outcome probabilities read in contiguous tiles, against numpy in 64 bits.
+"""Outcome probabilities read in contiguous tiles, and Grover loops applied as
+one affine map, against numpy in 64 bits.
 
-Tolerance: a probability is a sum of squares of total 1 accumulated with
-about 46 significant bits, inside the engine's parity bar of 1e-12
-(complex128).  complex64 squares exact FP32 values, so its probabilities meet
-the same bar against the rounded state."""
+Tolerances: a probability is a sum of squares of total 1 accumulated with
+about 46 significant bits, and a loop adds one FP64 offset to amplitudes of
+norm 1 whose sum is good to 2^-46 of the state's 1-norm; both stay inside the
+engine's parity bar of 1e-12 (complex128).  complex64 squares exact FP32
+values, so its probabilities meet the same bar against the rounded state."""
 from __future__ import annotations
 
 import numpy as np
@@ -11,6 +13,7 @@ import pytest
 
 from code_mojo_gb300 import butterfly as bfy
 from code_mojo_gb300 import workloads as W
+from tests.test_gpu_grover_loop import loop_body
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-12
@@ -47,3 +50,25 @@ def test_probabilities_of_any_register(n, dtype):
             values[k] = int(rng.integers(0, 2))
         assert np.max(np.abs(st.probabilities(q, values) - expected(z, n, q, values))) <= TOL
     st.close()
+
+
+def iterate(z, marked, iters):
+    for _ in range(iters):
+        for m in marked:
+            z[m] = -z[m]
+        z = 2 * z.mean() - z
+    return z
+
+
+# one CTA (12 qubits) against several (13, 15); odd and even counts; no, one,
+# eight and (at 3 qubits) every amplitude marked
+@pytest.mark.parametrize("n,marked", [(3, list(range(8))), (3, []), (5, [31]), (12, [0, 4095]), (13, [8191]),
+                                      (13, []), (15, [1, 2, 3, 500, 4096, 20000, 32766, 32767])])
+@pytest.mark.parametrize("iters", [2, 3, 70, 1001])
+def test_loop_is_the_repeated_iteration(n, marked, iters):
+    re, im = W.random_normal_state(n, 3 * n + iters)
+    st = bfy.QuantumState.from_soa(re, im)
+    bfy.execute(st, loop_body(n, marked, iters))
+    got = st.to_complex()
+    st.close()
+    assert np.max(np.abs(got - iterate(re + 1j * im, marked, iters))) <= TOL
