@@ -128,7 +128,7 @@ void upload_program_reserve(State& st, size_t ops) {
 // Everything a plan uploads: tile ops, and in the auxiliary buffer the
 // tensor-core passes' block descriptors, (at a 256-byte boundary) their
 // matrix images and destination tables, then (at a 16-byte boundary) the
-// unitary pool that the tile ops of dense unitaries index.
+// pool of unitary matrices and phase fans that tile ops index.
 struct Program {
   std::vector<TileOp> ops;
   std::vector<Blk5> blocks;
@@ -205,6 +205,7 @@ struct Step {
   uint64_t base = 0, modulus = 0;  // modexp: a (or a^-1 mod N) and N; a = n_exp
   bool digits = false;             // tensor-core pass in the complex128 digit form
   bool unitaries = false;          // tile pass: holds dense unitaries (GK_UNITARY ops)
+  bool fans = false;               // tile pass: holds phase fans
 };
 
 // a^-1 mod N for gcd(a, N) = 1 (extended Euclid, as modinv in algos/shor.mojo:46-53)
@@ -333,20 +334,19 @@ static void fused_pair_matrix(const bf_op& t0, const bf_op& t1, int& q_low, std:
 // per dense gate, beyond the 2.6 ms that moving the state costs either way).
 constexpr double kBlockUnits = 3.3;
 
-static double cuda_core_units(const TilePass& tp) {
+static double cuda_core_units(const std::vector<TileOp>& ops) {
   double u = 0;
-  for (const TileOp& t : tp.ops) {
+  for (const TileOp& t : ops) {
+    if (t.kind == GK_FAN) {
+      u += core_units(GK_FAN, 0);
+      continue;
+    }
     if (t.tloc < 0) {
       u += 0.4;  // diagonal gate on an outside target: one multiply per amplitude
       continue;
     }
-    switch (t.kind) {
-      case GK_SWAP: u += 0.5; break;
-      case GK_PHASE: u += 0.4; break;
-      case GK_DIAG: u += 0.6; break;
-      case GK_UNITARY: u += (double)(1 << (t.um - 1)); break;  // 2^m products per amplitude
-      default: u += 1.0; break;
-    }
+    u += core_units(t.kind, t.um);
+    if (t.fan) u += core_units(GK_FAN, 0);
   }
   return u;
 }
@@ -418,7 +418,9 @@ static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opt
       if (ps.is_tile && tensor && ps.tile.K == kBlockTileQubits && ps.tile.L == kTileLowQubits) {
         size_t b0 = pg.blocks.size(), i0 = pg.images.size(), o0 = pg.offsets.size();
         // the most blocks for which the block pass is still the cheaper form
-        const double cu = cuda_core_units(ps.tile);
+        std::vector<TileOp> merged;
+        merge_phases(ps.tile, merged, nullptr);
+        const double cu = cuda_core_units(merged);
         int max_blocks = 0;
         while (max_blocks < kMaxPassBlocks && (double)(max_blocks + 1) * block_units < cu) ++max_blocks;
         if (max_blocks > 0 &&
@@ -441,9 +443,11 @@ static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opt
         s.kind = Step::TILE;
         s.tile = ps.tile;
         s.prog_off = prog.size();
-        s.nprog = (int)ps.tile.ops.size();
-        for (const TileOp& t : ps.tile.ops) s.unitaries |= t.kind == GK_UNITARY;
-        prog.insert(prog.end(), ps.tile.ops.begin(), ps.tile.ops.end());
+        s.tile.ops.clear();
+        s.fans = merge_phases(ps.tile, s.tile.ops, &pg.umats) > 0;
+        s.nprog = (int)s.tile.ops.size();
+        for (const TileOp& t : s.tile.ops) s.unitaries |= t.kind == GK_UNITARY;
+        prog.insert(prog.end(), s.tile.ops.begin(), s.tile.ops.end());
         s.tile.ops.clear();
       } else if (ps.gate.kind == GK_UNITARY) {
         // a unitary the planner left on its own: its dense kernel
@@ -716,7 +720,9 @@ static void run_steps(State& st, const std::vector<Step>& steps, const Program& 
       case Step::GATE: launch_gate(st, s.gate); break;
       case Step::TILE:
         launch_tile_pass(st, st.d_prog + s.prog_off, s.nprog, s.tile,
-                         s.unitaries ? reinterpret_cast<const double*>(st.d_aux + pg.umats_offset()) : nullptr);
+                         s.unitaries || s.fans ? reinterpret_cast<const double*>(st.d_aux + pg.umats_offset())
+                                               : nullptr,
+                         s.unitaries, s.fans);
         break;
       case Step::TBLOCK:
         if (s.digits) {

@@ -15,6 +15,7 @@
 // replayed by bf_batch_run.
 #include <algorithm>
 #include <cstring>
+#include <map>
 #include <vector>
 
 #include "tile_body.cuh"
@@ -48,6 +49,7 @@ struct BatchDesc {
   const BatchTask* tasks;
   const BatchPass* passes;
   const TileOp* ops;
+  const double* fans;  // the phase fans' tables and constants
   unsigned int* done;
   unsigned long long* ticket;
   int* error;
@@ -55,7 +57,8 @@ struct BatchDesc {
   unsigned int spin_limit;
 };
 
-template <class P>
+// kFans: some pass holds phase fans (a separate form, as the tile kernel's)
+template <class P, bool kFans>
 __global__ void __launch_bounds__(kTileThreads) k_batch(const BatchDesc d) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned long long t_sh;
@@ -87,8 +90,8 @@ __global__ void __launch_bounds__(kTileThreads) k_batch(const BatchDesc d) {
       const BatchPass& bp = d.passes[task.pass];
       if (task.kind == TASK_TILE) {
         TileGeom geo = bp.geo;
-        run_tile<P, true>(static_cast<typename P::Glob*>(d.pool) + bp.offset, d.ops + bp.op_begin, (int)bp.nops,
-                          geo, task.tile, smem_raw);
+        run_tile<P, true, false, kFans>(static_cast<typename P::Glob*>(d.pool) + bp.offset, d.ops + bp.op_begin,
+                                        (int)bp.nops, geo, task.tile, smem_raw, d.fans);
       } else if constexpr (sizeof(typename P::Glob) == 8) {
         float2* base = reinterpret_cast<float2*>(d.pool) + bp.offset + ((uint64_t)task.tile << bp.geo.K);
         const int cnt = 1 << bp.geo.K;
@@ -155,6 +158,8 @@ struct Batch {
   BatchTask* d_tasks = nullptr;
   BatchPass* d_passes = nullptr;
   TileOp* d_ops = nullptr;
+  double* d_fans = nullptr;
+  bool fans = false;
   uint64_t* d_offsets = nullptr;
   unsigned int* d_done = nullptr;
   double* d_norm = nullptr;
@@ -188,6 +193,7 @@ static void enqueue_run(Batch& b) {
   d.tasks = b.d_tasks;
   d.passes = b.d_passes;
   d.ops = b.d_ops;
+  d.fans = b.d_fans;
   d.done = b.d_done;
   d.ticket = b.d_ticket;
   d.error = b.d_error;
@@ -203,7 +209,7 @@ static void enqueue_run(Batch& b) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  BF_CUDA(cudaLaunchKernelEx(&cfg, k_batch<P>, d));
+  BF_CUDA(cudaLaunchKernelEx(&cfg, b.fans ? k_batch<P, true> : k_batch<P, false>, d));
   BF_CUDA(cudaMemcpyAsync(b.h_error, b.d_error, sizeof(int), cudaMemcpyDeviceToHost, b.stream));
 }
 
@@ -222,11 +228,14 @@ template <class P>
 static void size_grid(Batch& b) {
   static PerDeviceOnce configured;  // one per instantiation of P
   configured.run(b.device, [] {
-    const size_t most = std::max<size_t>(tile_smem_bytes<P>(kMaxTileQubits, 0), kTileThreads * sizeof(double));
-    BF_CUDA(cudaFuncSetAttribute(k_batch<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    const size_t most =
+        std::max<size_t>(tile_smem_bytes<P>(kMaxTileQubits, 0, false, true), kTileThreads * sizeof(double));
+    BF_CUDA(cudaFuncSetAttribute(k_batch<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    BF_CUDA(cudaFuncSetAttribute(k_batch<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   });
   int per_sm = 0;
-  BF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<P>, kTileThreads, b.smem));
+  BF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b.fans ? k_batch<P, true> : k_batch<P, false>,
+                                                        kTileThreads, b.smem));
   if (per_sm < 1) fail(BF_EUNSUPPORTED, "batch kernel cannot be resident with %zu bytes of shared memory", b.smem);
   b.grid = (unsigned)(per_sm * b.num_sms);
 }
@@ -239,6 +248,7 @@ static void free_batch(Batch* b) {
   cudaFree(b->d_tasks);
   cudaFree(b->d_passes);
   cudaFree(b->d_ops);
+  cudaFree(b->d_fans);
   cudaFree(b->d_offsets);
   cudaFree(b->d_done);
   cudaFree(b->d_norm);
@@ -277,6 +287,8 @@ static Batch* build_batch(int ncirc, const int32_t* nq, const bf_op* const* ops,
     BF_CUDA(cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, b->device));
     std::vector<BatchPass> passes;
     std::vector<TileOp> prog;
+    std::vector<double> fan_pool;
+    std::map<std::pair<const bf_op*, std::pair<int64_t, int>>, int> planned;  // first circuit of each op list
     // per circuit: passes (each with its tile count)
     std::vector<std::vector<uint32_t>> circ_passes(ncirc);
     uint64_t off = 0;
@@ -284,6 +296,21 @@ static Batch* build_batch(int ncirc, const int32_t* nq, const bf_op* const* ops,
     for (int c = 0; c < ncirc; ++c) {
       int n = nq[c];
       if (n < 1 || n > 30) fail(BF_EINVAL, "circuit %d: num_qubits must be in [1, 30], got %d", c, n);
+      b->nq.push_back(n);
+      b->offsets.push_back(off);
+      off += ((1ull << n) + 31) & ~31ull;  // 256-byte aligned starts
+      // a circuit given again (the tuner repeats its sample) shares the ops,
+      // fans and geometry of its first plan
+      const auto known = planned.emplace(std::make_pair(ops[c], std::make_pair(nops[c], n)), c);
+      if (!known.second) {
+        for (uint32_t p : circ_passes[known.first->second]) {
+          BatchPass bp = passes[p];
+          bp.offset = b->offsets.back();
+          circ_passes[c].push_back((uint32_t)passes.size());
+          passes.push_back(bp);
+        }
+        continue;
+      }
       validate_ops(n, ops[c], nops[c]);
       std::vector<GateInstr> gates;
       for (int64_t i = 0; i < nops[c]; ++i) {
@@ -292,9 +319,6 @@ static Batch* build_batch(int ncirc, const int32_t* nq, const bf_op* const* ops,
           fail(BF_EUNSUPPORTED, "circuit %d: batches take gate transformations only (op %lld)", c, (long long)i);
         gates.push_back(lower_gate(op, o.specialized));
       }
-      b->nq.push_back(n);
-      b->offsets.push_back(off);
-      off += ((1ull << n) + 31) & ~31ull;  // 256-byte aligned starts
       int K = std::min(n, width_of_n[n]);
       for (auto& ps : plan_gates(n, gates, K, /*allow_single=*/false)) {
         BatchPass bp;
@@ -304,15 +328,16 @@ static Batch* build_batch(int ncirc, const int32_t* nq, const bf_op* const* ops,
         bp.geo.L = ps.tile.L;
         for (int j = 0; j < ps.tile.K; ++j) bp.geo.q[j] = ps.tile.q[j];
         bp.op_begin = (uint32_t)prog.size();
-        bp.nops = (uint32_t)ps.tile.ops.size();
-        prog.insert(prog.end(), ps.tile.ops.begin(), ps.tile.ops.end());
+        const bool fans = merge_phases(ps.tile, prog, &fan_pool) > 0;
+        b->fans |= fans;
+        bp.nops = (uint32_t)(prog.size() - bp.op_begin);
         circ_passes[c].push_back((uint32_t)passes.size());
         passes.push_back(bp);
         size_t sm = 0;
         switch (prec) {
-          case PREC_F64: sm = tile_smem_bytes<PolF64>(bp.geo.K, bp.geo.L); break;
-          case PREC_DF: sm = tile_smem_bytes<PolDF>(bp.geo.K, bp.geo.L); break;
-          default: sm = tile_smem_bytes<PolF32>(bp.geo.K, bp.geo.L); break;
+          case PREC_F64: sm = tile_smem_bytes<PolF64>(bp.geo.K, bp.geo.L, false, fans); break;
+          case PREC_DF: sm = tile_smem_bytes<PolDF>(bp.geo.K, bp.geo.L, false, fans); break;
+          default: sm = tile_smem_bytes<PolF32>(bp.geo.K, bp.geo.L, false, fans); break;
         }
         smem = std::max(smem, sm);
       }
@@ -347,6 +372,7 @@ static Batch* build_batch(int ncirc, const int32_t* nq, const bf_op* const* ops,
     dev_upload(&b->d_tasks, tasks);
     dev_upload(&b->d_passes, passes);
     dev_upload(&b->d_ops, prog);
+    dev_upload(&b->d_fans, fan_pool);
     dev_upload(&b->d_offsets, b->offsets);
     std::vector<unsigned int> zeros(ncirc, 0);
     dev_upload(&b->d_done, zeros);
@@ -406,7 +432,7 @@ constexpr int kTuneMinWidth = 8, kTuneMaxWidth = 12;
 
 template <class P>
 static size_t tile_smem_of(int K) {
-  return tile_smem_bytes<P>(K, std::min(K - 1, kTileLowQubits));
+  return tile_smem_bytes<P>(K, std::min(K - 1, kTileLowQubits), false, true);
 }
 
 static double time_batch(Batch& b) {

@@ -95,7 +95,8 @@ enum GKind : int32_t {
   GK_DIAG = 4,   // diag(d0, d1): m[0..1] = d0, m[6..7] = d1 (RZ)
   GK_RY = 5,     // real rotation [[c,-s],[s,c]]: m[0] = c, m[4] = s
   GK_DENSE_R = 6, // full 2x2 matrix whose m00 is real (m[1] == 0), as in every U3
-  GK_UNITARY = 7  // dense 2^um x 2^um matrix on qubits target .. target + um - 1
+  GK_UNITARY = 7, // dense 2^um x 2^um matrix on qubits target .. target + um - 1
+  GK_FAN = 8      // tile ops only: a phase fan on its own (below)
 };
 
 // Dense unitaries of up to this many qubits join fused runs (tile passes
@@ -148,8 +149,21 @@ struct TileOp {
   float mhl[16];
   int32_t um;         // GK_UNITARY: qubit count; 0 otherwise
   int32_t uoff;       // GK_UNITARY: offset (in doubles) of its matrix in the
-                      // program's unitary pool
+                      // program's pool
+  // The phase fan applied before the op (alone for GK_FAN): the product of
+  // the phases that share the centre qubit tloc, on the amplitudes whose
+  // centre bit is 1 (tloc < 0: the centre is in cmask_out, every amplitude).
+  // The phase of local index x is A[x mod 2^a] * B[x >> a] * c, with tables
+  // over the tile's low a and other K - a bits and c the product of the
+  // entries (mask, factor) whose outside qubits are all 1 in the CTA.
+  int32_t fan;        // 0: none; else 1 + its constant's slot in the pass
+  int32_t fan_off;    // offset (in doubles, even) in the program's pool:
+                      // A (2^a pairs), B (2^(K-a) pairs), the constants (mask bits, 0, re, im each)
+  int32_t fan_shape;  // a | kFanA (A is not all ones) | kFanB
+  int32_t fan_consts; // number of constants
 };
+constexpr int32_t kFanA = 1 << 8, kFanB = 1 << 9;
+constexpr int kMaxPassFans = 64;  // constants a pass keeps in shared memory
 
 struct TilePass {
   int32_t K;
@@ -322,8 +336,10 @@ void sync_state(State& st);
 // ---------------------------------------------------------------------------
 // Kernel launchers (device code lives in the .cu files).
 void launch_gate(State& s, const GateInstr& g);
-// d_umats: the device copy of the program's unitary pool (null without GK_UNITARY ops)
-void launch_tile_pass(State& s, const TileOp* d_ops, int nops, const TilePass& p, const double* d_umats = nullptr);
+// d_pool: the device copy of the program's pool (unitary matrices and phase
+// fans); unitaries / fans: the pass holds GK_UNITARY ops / phase fans
+void launch_tile_pass(State& s, const TileOp* d_ops, int nops, const TilePass& p, const double* d_pool = nullptr,
+                      bool unitaries = false, bool fans = false);
 void launch_block_pass(State& st, const Blk5* d_blocks, int nblocks, const unsigned char* d_images,
                        const uint16_t* d_offsets, const TilePass& p);
 // complex128 digit blocks (BLOCK_DIGITS); d_exp holds the scale exponent
@@ -392,6 +408,16 @@ struct PlanStep {
 // blocks run it faster than the double-float unitary kernel)
 std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int K, bool allow_single = true,
                                  double block_units = 0, double pass_cost = 2.5, bool keep_wide_unitaries = false);
+
+// A tile op's cost on the CUDA cores, in units of one dense gate over the tile
+// (um: qubits of a GK_UNITARY).
+double core_units(int kind, int um);
+// The ops of a CUDA-core tile pass with their phase gates merged into phase
+// fans (see TileOp): each phase waits until a gate acts non-diagonally on one
+// of its qubits, and the phases that meet that gate's target are multiplied
+// into one fan before it.  Tables go to `pool` (null: the ops only, for a
+// cost estimate).  Returns the number of fans.
+int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<double>* pool);
 
 // bf_execute's body on a prepared state; stream, event and SM count of a
 // state; releasing every buffer a state owns (api.cpp).

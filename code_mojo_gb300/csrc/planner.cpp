@@ -234,6 +234,175 @@ static TileOp to_tile_op(const GateInstr& g, const int* loc_of) {
   return t;
 }
 
+// ---- phase fans --------------------------------------------------------------
+// A phase gate of a tile pass, by the bits that must all be 1 (target among
+// them), inside and outside the tile.
+struct PhaseTerm {
+  const TileOp* op;
+  uint32_t loc;
+  uint64_t out;
+};
+
+// A fan needs at least this many phases: one alone touches a quarter or half
+// of the tile as its own op, a fan half of it with up to two products.
+constexpr int kMinFanTerms = 2;
+// tables stay below this many doubles (32-bit offsets); phases beyond it
+// remain ops of their own
+constexpr size_t kMaxFanPool = (size_t)1 << 30;
+
+// Whether a phase, its centre taken off, is a factor of the fan's tables (its
+// tile bits within one half) or of its constant (no tile bits).
+static bool fan_takes(const PhaseTerm& t, uint32_t centre_loc, uint64_t centre_out, int a) {
+  const uint32_t l = t.loc & ~centre_loc;
+  if (l == 0) return true;
+  if (t.out & ~centre_out) return false;
+  return (l >> a) == 0 || (l & ((1u << a) - 1u)) == 0;
+}
+
+// One table: entry x is the product of the factors whose mask is within x.
+static void fan_table(const std::vector<std::pair<uint32_t, const double*>>& terms, int bits, int shift, double* out) {
+  std::vector<double> one(2 * (size_t)bits, 0.0);  // product per single-bit mask
+  for (int b = 0; b < bits; ++b) one[2 * b] = 1.0;
+  auto mul = [](double* x, const double* f) {
+    const double r = x[0] * f[0] - x[1] * f[1];
+    x[1] = x[0] * f[1] + x[1] * f[0];
+    x[0] = r;
+  };
+  for (auto& t : terms) {
+    const uint32_t m = t.first >> shift;
+    if ((m & (m - 1)) == 0) mul(&one[2 * __builtin_ctz(m)], t.second);
+  }
+  out[0] = 1.0;
+  out[1] = 0.0;
+  for (int b = 0; b < bits; ++b)
+    for (uint32_t x = 0; x < (1u << b); ++x) {
+      double* d = out + 2 * ((1u << b) + x);
+      d[0] = out[2 * x];
+      d[1] = out[2 * x + 1];
+      mul(d, &one[2 * b]);
+    }
+  for (auto& t : terms) {
+    const uint32_t m = t.first >> shift;
+    if ((m & (m - 1)) == 0) continue;
+    for (uint32_t x = 0; x < (1u << bits); ++x)
+      if ((x & m) == m) mul(out + 2 * x, t.second);
+  }
+}
+
+int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<double>* pool) {
+  const int K = tp.K, a = K / 2;
+  std::vector<PhaseTerm> pending;
+  int fans = 0;
+  // fills op's fan from the terms around one centre
+  auto make_fan = [&](TileOp& op, const std::vector<PhaseTerm>& terms, uint32_t centre_loc) {
+    std::vector<std::pair<uint32_t, const double*>> ta, tb;
+    std::vector<const PhaseTerm*> consts;
+    for (const PhaseTerm& t : terms) {
+      const uint32_t l = t.loc & ~centre_loc;
+      if (l == 0) consts.push_back(&t);
+      else if ((l >> a) == 0) ta.emplace_back(l, t.op->m + 6);
+      else tb.emplace_back(l, t.op->m + 6);
+    }
+    op.fan = ++fans;
+    op.fan_shape = a | (ta.empty() ? 0 : kFanA) | (tb.empty() ? 0 : kFanB);
+    op.fan_consts = (int32_t)consts.size();
+    if (!pool) return;
+    op.fan_off = (int32_t)pool->size();
+    const size_t na = (size_t)1 << a, nb = (size_t)1 << (K - a);
+    pool->resize(pool->size() + 2 * (na + nb));
+    fan_table(ta, a, 0, pool->data() + op.fan_off);
+    fan_table(tb, K - a, a, pool->data() + op.fan_off + 2 * na);
+    for (const PhaseTerm* t : consts) {
+      double mask;
+      std::memcpy(&mask, &t->out, sizeof mask);
+      const double e[4] = {mask, 0.0, t->op->m[6], t->op->m[7]};
+      pool->insert(pool->end(), e, e + 4);
+    }
+    pool->push_back(1.0);  // the constants' product starts from here
+    pool->push_back(0.0);
+  };
+  // Emits terms as fans around the centre given (a tile bit) or, without
+  // one, around the qubit most of them share, the rest as ops of their own.
+  // `gate`: an uncontrolled single-target gate that a fan around its target
+  // can join; true when one did.
+  auto flush = [&](std::vector<PhaseTerm> terms, uint32_t centre, TileOp* gate) {
+    bool joined = false;
+    while ((int)terms.size() >= kMinFanTerms && fans < kMaxPassFans && (!pool || pool->size() < kMaxFanPool)) {
+      uint32_t cl = centre;
+      uint64_t co = 0;
+      if (!centre) {
+        int best = 0;
+        for (int q = 0; q < K + 64; ++q) {  // tile bits, then outside qubits
+          const uint32_t l = q < K ? 1u << q : 0u;
+          const uint64_t o = q < K ? 0ull : 1ull << (q - K);
+          int cnt = 0;
+          for (const PhaseTerm& t : terms)
+            cnt += ((t.loc & l) || (t.out & o)) && fan_takes(t, l, o, a);
+          if (cnt > best) {
+            best = cnt;
+            cl = l;
+            co = o;
+          }
+        }
+      }
+      std::vector<PhaseTerm> in, rest;
+      for (const PhaseTerm& t : terms) {
+        if (((t.loc & cl) || (t.out & co)) && fan_takes(t, cl, co, a)) in.push_back(t);
+        else rest.push_back(t);
+      }
+      if ((int)in.size() < kMinFanTerms) break;
+      if (gate && centre) {
+        make_fan(*gate, in, cl);
+        joined = true;
+      } else {
+        TileOp f;
+        std::memset(&f, 0, sizeof f);
+        f.kind = GK_FAN;
+        f.tloc = cl ? __builtin_ctz(cl) : -1;
+        f.tglob = cl ? tp.q[f.tloc] : __builtin_ctzll(co);
+        f.cmask_out = co;
+        make_fan(f, in, cl);
+        out.push_back(f);
+      }
+      terms.swap(rest);
+      if (centre) break;
+    }
+    for (const PhaseTerm& t : terms) out.push_back(*t.op);
+    return joined;
+  };
+  for (const TileOp& op : tp.ops) {
+    if (op.kind == GK_PHASE) {
+      PhaseTerm t;
+      t.op = &op;
+      t.loc = op.cmask_loc | (op.tloc >= 0 ? 1u << op.tloc : 0u);
+      t.out = op.cmask_out | (op.tloc < 0 ? 1ull << op.tglob : 0ull);
+      pending.push_back(t);
+      continue;
+    }
+    if (op.kind == GK_DIAG) {  // commutes with every phase
+      out.push_back(op);
+      continue;
+    }
+    const bool uni = op.kind == GK_UNITARY;
+    const uint32_t x = uni ? ((1u << op.um) - 1u) << op.tloc : 1u << op.tloc;
+    std::vector<PhaseTerm> met, rest;
+    for (const PhaseTerm& t : pending) (t.loc & x ? met : rest).push_back(t);
+    pending.swap(rest);
+    TileOp g = op;
+    const bool joins = !uni && op.kind != GK_SWAP && !op.cmask_loc && !op.cmask_out;
+    if (!met.empty()) flush(met, uni ? 0u : x, joins ? &g : nullptr);
+    out.push_back(g);
+  }
+  flush(pending, 0u, nullptr);
+  return fans;
+}
+
+// The work a tile pass counts a gate for when tiles are compared: a diagonal
+// gate joins any tile, and merges into a fan of whichever pass it runs in.
+static double gate_work(const GateInstr& g) {
+  return gate_bytes_fraction(g) * (gk_is_diagonal(g.kind) ? 0.02 : 1.0);
+}
+
 // The work (per-gate bytes, in units of S) a tile pass over the qubit set
 // inQ takes from the remaining gates: a gate joins when its non-diagonal
 // target is in the set and it commutes with every gate deferred before it.
@@ -244,7 +413,7 @@ static double pass_work(const std::vector<const GateInstr*>& remaining, uint64_t
     const uint64_t Xg = gate_xmask(*g);
     const uint64_t Ag = gate_amask(*g);
     if (!(Xg & blockedAll) && !(Ag & blockedX) && !(Xg & ~inQ)) {
-      w += gate_bytes_fraction(*g);
+      w += gate_work(*g);
     } else {
       blockedX |= Xg;
       blockedAll |= Ag;
@@ -295,14 +464,13 @@ static int pass_blocks(const std::vector<const GateInstr*>& remaining, uint64_t 
 }
 
 // The CUDA-core tile kernel's cost of the gates a pass over inQ takes, in
-// dense-gate units (dense 1, exchange 0.5, phase 0.4, other diagonal 0.6, a
-// diagonal gate on an outside target 0.4, an m-qubit unitary 2^(m-1): its
-// 2^m complex products per amplitude against a dense gate's 2).
+// dense-gate units (core_units of the same gates), its phases merged into
+// fans and those no gate of the pass meets left to a later one.
 static double pass_core_units(const std::vector<const GateInstr*>& remaining, uint64_t inQ, uint64_t all) {
   uint64_t blockedX = 0, blockedAll = 0;
   double u = 0;
+  std::vector<uint64_t> pending;
   for (const GateInstr* g : remaining) {
-    const uint64_t tb = 1ull << g->target;
     const uint64_t Xg = gate_xmask(*g);
     const uint64_t Ag = gate_amask(*g);
     if ((Xg & blockedAll) || (Ag & blockedX) || (Xg & ~inQ)) {
@@ -311,14 +479,38 @@ static double pass_core_units(const std::vector<const GateInstr*>& remaining, ui
       if ((blockedX & all) == all) break;
       continue;
     }
-    if (g->kind == GK_UNITARY) u += (double)(1 << (g->um - 1));
-    else if (!(tb & inQ)) u += 0.4;
-    else if (g->kind == GK_SWAP) u += 0.5;
-    else if (g->kind == GK_PHASE) u += 0.4;
-    else if (g->kind == GK_DIAG) u += 0.6;
-    else u += 1.0;
+    if (g->kind == GK_PHASE) {
+      pending.push_back(Ag);
+      continue;
+    }
+    u += core_units(g->kind, g->um);
+    if (!Xg) continue;
+    size_t kept = 0, met = 0;
+    for (uint64_t p : pending) {
+      if (p & Xg) ++met;
+      else pending[kept++] = p;
+    }
+    pending.resize(kept);
+    if (met >= (size_t)kMinFanTerms) u += core_units(GK_FAN, 0);
+    else if (met) u += core_units(GK_PHASE, 0);
   }
   return u;
+}
+
+// A tile op's cost on the CUDA cores, in units of one dense gate over the
+// tile (double-float: about 134 instructions per pair, a Hadamard 86, a fan
+// 76 on its half of the amplitudes; an m-qubit unitary does 2^m complex
+// products per amplitude against a dense gate's 2).
+double core_units(int kind, int um) {
+  switch (kind) {
+    case GK_SWAP: return 0.5;
+    case GK_PHASE: return 0.4;
+    case GK_DIAG: return 0.6;
+    case GK_H: return 0.65;
+    case GK_FAN: return 0.6;
+    case GK_UNITARY: return (double)(1 << (um - 1));
+    default: return 1.0;
+  }
 }
 
 std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int K, bool allow_single,
@@ -367,6 +559,7 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
         }
       }
     }
+    bool blocks_chosen = false;
     if (nQ == K && K < n) {
       uint64_t targets = 0;
       for (const GateInstr* g : remaining) targets |= gate_xmask(*g);
@@ -394,7 +587,6 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
       };
       auto work = [&](uint64_t set) { return pass_work(remaining, set, all); };
       const uint64_t start = inQ;
-      bool chosen = false;
       const uint64_t by_work = search(start, work);
       if (block_units > 0) {
         // Passes that may run as tensor-core blocks: the tile that takes the
@@ -409,12 +601,13 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
         const double core_rate = work(by_work) / (pass_cost + pass_core_units(remaining, by_work, all) / block_units);
         if ((double)pass_blocks(remaining, set, all) * block_units < core && block_rate(set) >= core_rate) {
           inQ = set;
-          chosen = true;
+          blocks_chosen = true;
         }
       }
-      if (!chosen) inQ = by_work;
+      if (!blocks_chosen) inQ = by_work;
     }
     std::vector<const GateInstr*> taken, deferred;
+    std::vector<size_t> taken_at, deferred_at;  // their places in `remaining`
     {
       uint64_t blockedX = 0, blockedAll = 0;
       size_t i = 0;
@@ -424,8 +617,10 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
         const uint64_t Ag = gate_amask(*g);
         if (!(Xg & blockedAll) && !(Ag & blockedX) && !(Xg & ~inQ)) {
           taken.push_back(g);
+          taken_at.push_back(i);
         } else {
           deferred.push_back(g);
+          deferred_at.push_back(i);
           blockedX |= Xg;
           blockedAll |= Ag;
           if ((blockedX & all) == all) {
@@ -434,7 +629,45 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
           }
         }
       }
-      deferred.insert(deferred.end(), remaining.begin() + (std::ptrdiff_t)i, remaining.end());
+      for (; i < remaining.size(); ++i) {
+        deferred.push_back(remaining[i]);
+        deferred_at.push_back(i);
+      }
+    }
+    // A phase that no gate of this pass meets goes back when a deferred gate
+    // acts non-diagonally on one of its qubits: there it joins a fan that
+    // pass applies anyway (20-qubit QFT: no fan of its own in any pass).  A
+    // tile chosen for tensor-core blocks keeps it, as part of a block.
+    if (!blocks_chosen) {
+      uint64_t later = 0, met = 0;
+      for (const GateInstr* g : deferred) later |= gate_xmask(*g);
+      std::vector<char> back(taken.size(), 0);
+      bool any = false;
+      for (size_t k = taken.size(); k-- > 0;) {
+        const uint64_t Xg = gate_xmask(*taken[k]);
+        met |= Xg;
+        if (taken[k]->kind != GK_PHASE) continue;
+        const uint64_t Ag = gate_amask(*taken[k]);
+        back[k] = !(Ag & met) && (Ag & later);
+        any |= back[k] != 0;
+      }
+      if (any) {
+        std::vector<const GateInstr*> keep, merged;
+        size_t d = 0;
+        for (size_t k = 0; k < taken.size(); ++k) {
+          if (!back[k]) {
+            keep.push_back(taken[k]);
+            continue;
+          }
+          while (d < deferred.size() && deferred_at[d] < taken_at[k]) merged.push_back(deferred[d++]);
+          merged.push_back(taken[k]);
+        }
+        merged.insert(merged.end(), deferred.begin() + (std::ptrdiff_t)d, deferred.end());
+        if (!keep.empty()) {
+          taken.swap(keep);
+          deferred.swap(merged);
+        }
+      }
     }
     if (taken.empty()) fail(BF_EINVAL, "internal: tile planner made no progress (K=%d, n=%d)", K, n);
     double single_bytes = 0;

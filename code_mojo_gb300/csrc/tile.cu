@@ -21,19 +21,36 @@
 
 namespace bf {
 
-// kUnitaries: the pass holds dense unitaries (a separate form, so that
-// passes without them keep the gate loop's small register count)
-template <class P, bool kUnitaries>
+// kUnitaries: the pass holds dense unitaries; kFans: phase fans (separate
+// forms, so that passes without them keep the gate loop's small register
+// count and shared memory)
+template <class P, bool kUnitaries, bool kFans>
 __global__ void __launch_bounds__(kTileThreads) k_tile(typename P::Glob* __restrict__ s,
                                                        const TileOp* __restrict__ ops, int nops,
-                                                       const TileGeom geo, const double* __restrict__ umats) {
+                                                       const TileGeom geo, const double* __restrict__ pool) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  run_tile<P, false, kUnitaries>(s, ops, nops, geo, blockIdx.x, smem_raw, umats);
+  run_tile<P, false, kUnitaries, kFans>(s, ops, nops, geo, blockIdx.x, smem_raw, pool);
 }
 
+template <class P, bool kUnitaries, bool kFans>
+static void launch_tile_form(State& st, const TileOp* d_ops, int nops, const TileGeom& geo, const double* d_pool) {
+  static PerDeviceOnce configured;  // one per instantiation
+  configured.run(st.device, [] {
+    BF_CUDA(cudaFuncSetAttribute(k_tile<P, kUnitaries, kFans>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)tile_smem_bytes<P>(kMaxTileQubits, 0, kUnitaries, kFans)));
+  });
+  const uint64_t blocks = st.N >> geo.K;
+  if (blocks > 0x7fffffffull) fail(BF_EUNSUPPORTED, "tile grid too large");
+  k_tile<P, kUnitaries, kFans><<<(unsigned)blocks, kTileThreads,
+                                 tile_smem_bytes<P>(geo.K, geo.L, kUnitaries, kFans), st.stream>>>(
+      static_cast<typename P::Glob*>(st.amp), d_ops, nops, geo, d_pool);
+  BF_CUDA(cudaGetLastError());
+  st.launches++;
+}
 
 template <class P>
-static void launch_tile_p(State& st, const TileOp* d_ops, int nops, const TilePass& p, const double* d_umats) {
+static void launch_tile_p(State& st, const TileOp* d_ops, int nops, const TilePass& p, const double* d_pool,
+                          bool unitaries, bool fans) {
   TileGeom geo;
   geo.K = p.K;
   geo.L = p.L;
@@ -41,29 +58,18 @@ static void launch_tile_p(State& st, const TileOp* d_ops, int nops, const TilePa
   for (int j = 0; j < p.K; ++j) geo.q[j] = p.q[j];
   for (int j = 0; j < geo.L; ++j)
     if (geo.q[j] != j) fail(BF_EINVAL, "internal: tile qubits must start with 0..%d", geo.L - 1);
-  const bool uni = d_umats != nullptr;
-  size_t smem = tile_smem_bytes<P>(p.K, geo.L, uni);
-  static PerDeviceOnce configured;  // one per instantiation of P
-  configured.run(st.device, [] {
-    BF_CUDA(cudaFuncSetAttribute(k_tile<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tile_smem_bytes<P>(kMaxTileQubits, 0)));
-    BF_CUDA(cudaFuncSetAttribute(k_tile<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tile_smem_bytes<P>(kMaxTileQubits, 0, true)));
-  });
-  uint64_t blocks = st.N >> p.K;
-  if (blocks > 0x7fffffffull) fail(BF_EUNSUPPORTED, "tile grid too large");
-  auto* amp = static_cast<typename P::Glob*>(st.amp);
-  if (uni) k_tile<P, true><<<(unsigned)blocks, kTileThreads, smem, st.stream>>>(amp, d_ops, nops, geo, d_umats);
-  else k_tile<P, false><<<(unsigned)blocks, kTileThreads, smem, st.stream>>>(amp, d_ops, nops, geo, nullptr);
-  BF_CUDA(cudaGetLastError());
-  st.launches++;
+  if (unitaries && fans) launch_tile_form<P, true, true>(st, d_ops, nops, geo, d_pool);
+  else if (unitaries) launch_tile_form<P, true, false>(st, d_ops, nops, geo, d_pool);
+  else if (fans) launch_tile_form<P, false, true>(st, d_ops, nops, geo, d_pool);
+  else launch_tile_form<P, false, false>(st, d_ops, nops, geo, d_pool);
 }
 
-void launch_tile_pass(State& st, const TileOp* d_ops, int nops, const TilePass& p, const double* d_umats) {
+void launch_tile_pass(State& st, const TileOp* d_ops, int nops, const TilePass& p, const double* d_pool,
+                      bool unitaries, bool fans) {
   switch (st.prec) {
-    case PREC_F64: launch_tile_p<PolF64>(st, d_ops, nops, p, d_umats); break;
-    case PREC_DF: launch_tile_p<PolDF>(st, d_ops, nops, p, d_umats); break;
-    default: launch_tile_p<PolF32>(st, d_ops, nops, p, d_umats); break;
+    case PREC_F64: launch_tile_p<PolF64>(st, d_ops, nops, p, d_pool, unitaries, fans); break;
+    case PREC_DF: launch_tile_p<PolDF>(st, d_ops, nops, p, d_pool, unitaries, fans); break;
+    default: launch_tile_p<PolF32>(st, d_ops, nops, p, d_pool, unitaries, fans); break;
   }
 }
 

@@ -2,6 +2,8 @@
 // tile kernel (tile.cu) and the batched persistent kernel (batch.cu).
 #pragma once
 
+#include <cstring>
+
 #include "amp_math.cuh"
 #include "bf_internal.h"
 
@@ -57,6 +59,64 @@ __device__ __forceinline__ void tile_gate(int kind, typename P::Smem* amp, int T
     case GK_DIAG: tile_pairs<P, GK_DIAG, kCtl>(amp, TS, tloc, cml, g); break;
     case GK_DENSE_R: tile_pairs<P, GK_DENSE_R, kCtl>(amp, TS, tloc, cml, g); break;
     default: tile_pairs<P, GK_RY, kCtl>(amp, TS, tloc, cml, g); break;
+  }
+}
+
+// Phase fans.  Bound by FP32 issue (double-float) and by the shared-memory
+// round trip per op (complex64), so what a phase costs is its pass over the
+// tile: as an op of its own it reads, multiplies and writes a quarter or half
+// of it behind a barrier.  The n(n-1)/2 phases of a Fourier transform become
+// at most one fan per Hadamard, multiplied into the pair the Hadamard has in
+// registers anyway: one or two complex products per pair whatever the number
+// of phases.  At 24 qubits, complex128, the value encoding (24 P, 276 CP, 48
+// H) took 4.13 ms as 46 digit blocks in 4 passes and takes 2.25 ms in 3 tile
+// passes with fans; at 27 qubits, complex64, 17.3 against 6.8 ms; the 20-qubit
+// QFT's passes, complex128, 0.30 against 0.15 ms.
+//
+// A phase fan as the CTA holds it: tables in shared memory (the constant
+// folded into one of them), or with neither table the constant alone.
+template <class P>
+struct FanView {
+  const typename P::Smem* A;
+  const typename P::Smem* B;
+  uint32_t amask;
+  int abits;
+  bool use_a, use_b;
+  typename P::R c;
+};
+
+template <class P>
+__device__ __forceinline__ typename P::R cmul_r(typename P::R x, const typename P::R& w) {
+  P::cmul_by(x, w.re, w.im);
+  return x;
+}
+
+template <class P>
+__device__ __forceinline__ typename P::R fan_apply(const FanView<P>& f, typename P::R v, uint32_t i) {
+  if (f.use_a) v = cmul_r<P>(v, P::from_smem(f.A[i & f.amask]));
+  if (f.use_b) v = cmul_r<P>(v, P::from_smem(f.B[i >> f.abits]));
+  if (!f.use_a && !f.use_b) v = cmul_r<P>(v, f.c);
+  return v;
+}
+
+// One uncontrolled in-tile gate with a fan on its target: the fan multiplies
+// the pair's second amplitude on its way into the gate (GK_FAN: alone).
+template <class P, int KIND>
+__device__ __forceinline__ void tile_pairs_fan(typename P::Smem* amp, int TS, int tloc, const typename P::Coef& g,
+                                               const FanView<P>& f) {
+  using R = typename P::R;
+  const uint32_t low = (1u << tloc) - 1u, tb = 1u << tloc;
+#pragma unroll 1
+  for (int p = threadIdx.x; p < (TS >> 1); p += kTileThreads) {
+    const uint32_t i0 = (((uint32_t)p & ~low) << 1) | ((uint32_t)p & low);
+    const uint32_t i1 = i0 | tb;
+    R v = fan_apply<P>(f, P::from_smem(amp[i1]), i1);
+    if (KIND != GK_FAN) {
+      R u = P::from_smem(amp[i0]);
+      apply_pair<P>(KIND, u, v, g);
+      amp[i0] = P::to_smem(u);
+    }
+    amp[i1] = P::to_smem(v);
   }
 }
 
@@ -132,6 +192,13 @@ __host__ __device__ inline size_t tile_umat_offset(int K, int L) {
          ~(size_t)15;
 }
 
+// shared memory of the fans: the pass's constants, then the current op's
+// tables (2^a + 2^(K-a) entries, a = K / 2)
+template <class P>
+__host__ __device__ inline size_t tile_fan_bytes(int K) {
+  return (kMaxPassFans + ((size_t)1 << (K / 2)) + ((size_t)1 << (K - K / 2))) * sizeof(typename P::Smem);
+}
+
 // One tile: load the 2^K amplitudes of tile `tile` (the non-tile qubits set
 // to the bits of `tile`), apply ops[0..nops) in shared memory, store.  Called
 // by every thread of a CTA of kTileThreads threads; `smem_raw` holds
@@ -141,12 +208,14 @@ __host__ __device__ inline size_t tile_umat_offset(int K, int L) {
 // across SMs); a separate launch per pass does not need it.
 // kUnitaries: the ops may include GK_UNITARY (their register-heavy loop is
 // compiled only into this form; passes without them keep the lean one);
-// umats is then the unitary pool (row-major interleaved FP64), and
-// `smem_raw` also holds the staged matrix (tile_smem_bytes(K, L, true)).
-template <class P, bool kL2Loads = false, bool kUnitaries = false>
+// pool then holds their matrices (row-major interleaved FP64), and
+// `smem_raw` also holds the staged matrix.
+// kFans: the ops may carry phase fans; pool then holds their tables and
+// constants, and `smem_raw` also holds the staged ones (tile_smem_bytes).
+template <class P, bool kL2Loads = false, bool kUnitaries = false, bool kFans = false>
 __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const TileOp* __restrict__ ops, int nops,
                                          const TileGeom& geo, uint64_t tile, unsigned char* smem_raw,
-                                         const double* __restrict__ umats = nullptr) {
+                                         const double* __restrict__ pool = nullptr) {
   using R = typename P::R;
   using S = typename P::Smem;
   const int K = geo.K, L = geo.L;
@@ -169,6 +238,44 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
   }
   __syncthreads();
 
+  auto pool_at = [&](const double* d) {
+    typename P::Glob gv;
+    if constexpr (sizeof(typename P::Glob) == 16) gv = __ldg(reinterpret_cast<const double2*>(d));
+    else gv = make_float2((float)__ldg(d), (float)__ldg(d + 1));
+    return P::from_glob(gv);
+  };
+  S* fan_c = reinterpret_cast<S*>(smem_raw + tile_umat_offset<P>(K, L) +
+                                  (kUnitaries ? ((size_t)1 << (2 * kTileUnitaryMax)) * sizeof(S) : 0));
+  S* fan_a = fan_c + kMaxPassFans;
+  if constexpr (kFans) {
+    // the fans' constants for this CTA's outside bits, one warp per fan: the
+    // lanes' factors multiplied by butterfly shuffles
+    const int lane = tid & 31;
+    for (int i = tid >> 5; i < nops; i += kTileThreads / 32) {
+      const int slot = __ldg(&ops[i].fan), nc = __ldg(&ops[i].fan_consts);
+      if (slot == 0 || nc == 0) continue;
+      const double* c = pool + __ldg(&ops[i].fan_off) + 2 * ((1 << (K / 2)) + (1 << (K - K / 2)));
+      R acc = pool_at(c + 4 * nc);  // one
+      for (int k = lane; k < nc; k += 32) {
+        const uint64_t m = (uint64_t)__double_as_longlong(__ldg(c + 4 * k));
+        if ((obase & m) == m) acc = cmul_r<P>(acc, pool_at(c + 4 * k + 2));
+      }
+      int span = 1;
+      while (span < nc && span < 32) span <<= 1;
+      for (int off = span >> 1; off > 0; off >>= 1) {
+        S o = P::to_smem(acc), r;
+        constexpr int kWords = sizeof(S) / 4;
+        unsigned int w[kWords], x[kWords];
+        memcpy(w, &o, sizeof o);
+#pragma unroll
+        for (int q = 0; q < kWords; ++q) x[q] = __shfl_xor_sync(0xffffffffu, w[q], off);
+        memcpy(&r, x, sizeof r);
+        acc = cmul_r<P>(acc, P::from_smem(r));
+      }
+      if (lane == 0) fan_c[slot - 1] = P::to_smem(acc);
+    }
+  }
+
   const int lowmask = (1 << L) - 1;
   for (int e = tid; e < TS; e += kTileThreads) {
     uint64_t gi = obase | (uint64_t)(e & lowmask) | hoff[e >> L];
@@ -186,7 +293,7 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
     if (kUnitaries && kind == GK_UNITARY) {
       // stage the matrix, then every group of the tile
       const int um = __ldg(&op->um);
-      const double* u = umats + __ldg(&op->uoff);
+      const double* u = pool + __ldg(&op->uoff);
       S* mat = reinterpret_cast<S*>(smem_raw + tile_umat_offset<P>(K, L));
       const int dim = 1 << um;
       for (int e = tid; e < dim * dim; e += kTileThreads) {
@@ -220,7 +327,40 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
       continue;
     }
     const typename P::Coef g = P::coef(op->m, op->mhl);
-    if (tloc >= 0) {
+    if (kFans && __ldg(&op->fan) != 0) {
+      const int shape = __ldg(&op->fan_shape), nc = __ldg(&op->fan_consts);
+      FanView<P> f;
+      f.use_a = (shape & kFanA) != 0;
+      f.use_b = (shape & kFanB) != 0;
+      f.abits = K / 2;
+      f.amask = (1u << f.abits) - 1u;
+      f.A = fan_a;
+      f.B = fan_a + (1 << f.abits);
+      const S* cs = fan_c + (__ldg(&op->fan) - 1);
+      if (f.use_a || f.use_b) {
+        // the tables, the constant folded into B (or the only table)
+        const int na = 1 << f.abits, nt = na + (1 << (K - f.abits));
+        if (tid < nt && (tid < na ? f.use_a : f.use_b)) {
+          R w = pool_at(pool + __ldg(&op->fan_off) + 2 * tid);
+          if (nc && (tid >= na || !f.use_b)) w = cmul_r<P>(w, P::from_smem(*cs));
+          fan_a[tid] = P::to_smem(w);
+        }
+        __syncthreads();
+      } else {
+        f.c = P::from_smem(*cs);
+      }
+      if (tloc < 0) {  // the centre is outside the tile (and set): every amplitude
+        for (int e = tid; e < TS; e += kTileThreads) amp[e] = P::to_smem(fan_apply<P>(f, P::from_smem(amp[e]), e));
+      } else {
+        switch (kind) {
+          case GK_FAN: tile_pairs_fan<P, GK_FAN>(amp, TS, tloc, g, f); break;
+          case GK_H: tile_pairs_fan<P, GK_H>(amp, TS, tloc, g, f); break;
+          case GK_DENSE_R: tile_pairs_fan<P, GK_DENSE_R>(amp, TS, tloc, g, f); break;
+          case GK_RY: tile_pairs_fan<P, GK_RY>(amp, TS, tloc, g, f); break;
+          default: tile_pairs_fan<P, GK_DENSE>(amp, TS, tloc, g, f); break;
+        }
+      }
+    } else if (tloc >= 0) {
       if (cml) tile_gate<P, true>(kind, amp, TS, tloc, cml, g);
       else tile_gate<P, false>(kind, amp, TS, tloc, 0u, g);
     } else {
@@ -246,12 +386,14 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
 }
 
 // shared memory of run_tile; with_unitary: room for a staged
-// 2^kTileUnitaryMax-square matrix
+// 2^kTileUnitaryMax-square matrix; with_fans: for the phase fans
 template <class P>
-inline size_t tile_smem_bytes(int K, int L, bool with_unitary = false) {
-  if (with_unitary)
-    return tile_umat_offset<P>(K, L) + ((size_t)1 << (2 * kTileUnitaryMax)) * sizeof(typename P::Smem);
-  return ((size_t)1 << K) * sizeof(typename P::Smem) + ((size_t)1 << (K - L)) * sizeof(uint64_t);
+inline size_t tile_smem_bytes(int K, int L, bool with_unitary = false, bool with_fans = false) {
+  if (!with_unitary && !with_fans)
+    return ((size_t)1 << K) * sizeof(typename P::Smem) + ((size_t)1 << (K - L)) * sizeof(uint64_t);
+  return tile_umat_offset<P>(K, L) +
+         (with_unitary ? ((size_t)1 << (2 * kTileUnitaryMax)) * sizeof(typename P::Smem) : 0) +
+         (with_fans ? tile_fan_bytes<P>(K) : 0);
 }
 
 }  // namespace bf
