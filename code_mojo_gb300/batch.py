@@ -41,7 +41,9 @@ class Batch:
         re = np.empty(1 << n)
         im = np.empty(1 << n)
         F.check(F.lib().bf_batch_download(self._h, c, re.ctypes.data, im.ctypes.data))
-        return re + 1j * im
+        z = np.empty(1 << n, dtype=np.complex128)
+        z.real, z.imag = re, im
+        return z
 
     def stats(self) -> dict:
         t, p, g = C.c_int64(), C.c_int64(), C.c_int32()

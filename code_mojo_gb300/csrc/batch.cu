@@ -171,6 +171,8 @@ struct Batch {
   cudaStream_t stream = nullptr;
   cudaGraphExec_t graph = nullptr;
   uint64_t launches = 0;
+  HostStage host_stage;
+  std::mutex download_mutex;  // the staging's user
   // autotuning record: per qubit count, the candidate tile widths timed on a
   // sample of the batch's circuits of that size, and the width chosen
   std::vector<BatchTuneRow> tuning;
@@ -255,6 +257,7 @@ static void free_batch(Batch* b) {
   cudaFree(b->d_ticket);
   cudaFree(b->d_error);
   if (b->h_error) cudaFreeHost(b->h_error);
+  b->host_stage.release();
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }
@@ -565,25 +568,19 @@ void batch_sync(Batch& b) {
   if (*b.h_error) fail(BF_ETIMEDOUT, "batch: a task waited past its bound for its circuit's previous pass");
 }
 
+// Through the pinned staging: one conversion kernel and one host copy for a
+// circuit of up to 2^19 amplitudes.  Several threads may download at once.
 void batch_download(Batch& b, int c, double* re, double* im) {
   if (c < 0 || c >= b.ncirc) fail(BF_EINVAL, "circuit index %d out of range", c);
   batch_sync(b);
-  uint64_t N = 1ull << b.nq[c];
-  size_t eb = b.amp_bytes();
-  std::vector<unsigned char> h(N * eb);
-  BF_CUDA(cudaMemcpy(h.data(), static_cast<unsigned char*>(b.pool) + b.offsets[c] * eb, N * eb,
-                     cudaMemcpyDeviceToHost));
-  for (uint64_t i = 0; i < N; ++i) {
-    if (eb == 16) {
-      const double* p = reinterpret_cast<const double*>(h.data()) + 2 * i;
-      re[i] = p[0];
-      im[i] = p[1];
-    } else {
-      const float* p = reinterpret_cast<const float*>(h.data()) + 2 * i;
-      re[i] = (double)p[0];
-      im[i] = (double)p[1];
-    }
-  }
+  const uint64_t N = 1ull << b.nq[c];
+  const size_t eb = b.amp_bytes();
+  const char* amps = static_cast<const char*>(b.pool) + b.offsets[c] * eb;
+  auto convert = [&](double* r, double* i, uint64_t off, uint64_t cnt) {
+    launch_deinterleave(amps + off * eb, b.dtype, r, i, cnt, b.num_sms, b.stream);
+  };
+  std::lock_guard<std::mutex> one(b.download_mutex);
+  b.host_stage.download(N, re, im, b.stream, convert);
 }
 
 void batch_destroy(Batch* b) { free_batch(b); }

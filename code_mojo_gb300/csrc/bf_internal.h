@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -243,6 +244,22 @@ void block_image(const double* u, unsigned char* img);
 // ---------------------------------------------------------------------------
 struct PlanCache;  // a state's recent plans (api.cpp)
 
+// Two pinned chunk buffers (re and im each) that conversion kernels write as
+// mapped memory on their way to pageable host arrays.  One owner and one
+// stream; one download at a time.
+constexpr uint64_t kHostChunk = 1ull << 19;  // amplitudes of a chunk at most
+struct HostStage {
+  // launches the conversion of amplitudes [off, off + cnt) of the transfer
+  // to (re, im) on the owner's stream
+  using Convert = std::function<void(double* re, double* im, uint64_t off, uint64_t cnt)>;
+  double* p = nullptr;
+  uint64_t cap = 0;                          // amplitudes per buffer
+  cudaEvent_t done[2] = {nullptr, nullptr};  // the last kernel on buffer k
+  // blocks until re and im hold `count` amplitudes
+  void download(uint64_t count, double* re, double* im, cudaStream_t stream, const Convert& convert);
+  void release();
+};
+
 // The device state.
 struct State {
   int32_t n = 0;
@@ -275,6 +292,8 @@ struct State {
   // caller's arrays and these while the DMA engine moves the other buffer
   void* h_stage = nullptr;
   size_t h_stage_bytes = 0;
+  // pinned staging for smaller downloads into pageable arrays
+  HostStage host_stage;
   // dense unitary matrix (device copy of the current op's matrix)
   double* d_umat = nullptr;
   // norms before / after a complex64 circuit and the rescale factor
@@ -365,6 +384,9 @@ void launch_unitary(State& s, const double* h_u, int target, int m, int control)
 void launch_set_basis(State& s, uint64_t idx);
 void launch_interleave(State& s, const double* d_re, const double* d_im, uint64_t off, uint64_t cnt);
 void launch_deinterleave(State& s, double* d_re, double* d_im, uint64_t off, uint64_t cnt);
+// amps (dtype BF_C128 or BF_C64) -> re, im on `stream`
+void launch_deinterleave(const void* amps, int dtype, double* d_re, double* d_im, uint64_t cnt, int num_sms,
+                         cudaStream_t stream);
 double reduce_norm2(State& s);
 // <a|b> = sum conj(a_i) b_i (states of equal size, either dtype); synchronises a
 void inner_product(State& a, State& b, double* re, double* im);

@@ -56,9 +56,10 @@ __global__ void __launch_bounds__(256) k_deinterleave_c64(const float2* __restri
   }
 }
 
-static unsigned grid_for(const State& st, uint64_t cnt) {
-  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((cnt + 255) / 256, (uint64_t)st.num_sms * 16));
+static unsigned grid_for(int num_sms, uint64_t cnt) {
+  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((cnt + 255) / 256, (uint64_t)num_sms * 16));
 }
+static unsigned grid_for(const State& st, uint64_t cnt) { return grid_for(st.num_sms, cnt); }
 
 void launch_interleave(State& st, const double* d_re, const double* d_im, uint64_t off, uint64_t cnt) {
   if (st.dtype == BF_C128)
@@ -69,14 +70,19 @@ void launch_interleave(State& st, const double* d_re, const double* d_im, uint64
   st.launches++;
 }
 
-void launch_deinterleave(State& st, double* d_re, double* d_im, uint64_t off, uint64_t cnt) {
-  if (st.dtype == BF_C128)
-    k_deinterleave_c128<<<grid_for(st, cnt), 256, 0, st.stream>>>(static_cast<const double2*>(st.amp) + off, d_re,
-                                                                   d_im, cnt);
+void launch_deinterleave(const void* amps, int dtype, double* d_re, double* d_im, uint64_t cnt, int num_sms,
+                         cudaStream_t stream) {
+  const unsigned grid = grid_for(num_sms, cnt);
+  if (dtype == BF_C128)
+    k_deinterleave_c128<<<grid, 256, 0, stream>>>(static_cast<const double2*>(amps), d_re, d_im, cnt);
   else
-    k_deinterleave_c64<<<grid_for(st, cnt), 256, 0, st.stream>>>(static_cast<const float2*>(st.amp) + off, d_re,
-                                                                  d_im, cnt);
+    k_deinterleave_c64<<<grid, 256, 0, stream>>>(static_cast<const float2*>(amps), d_re, d_im, cnt);
   BF_CUDA(cudaGetLastError());
+}
+
+void launch_deinterleave(State& st, double* d_re, double* d_im, uint64_t off, uint64_t cnt) {
+  launch_deinterleave(static_cast<const char*>(st.amp) + off * st.amp_bytes(), st.dtype, d_re, d_im, cnt, st.num_sms,
+                      st.stream);
   st.launches++;
 }
 
