@@ -156,9 +156,10 @@ __device__ __forceinline__ dfl df_from_double(double x) {
   return r;
 }
 
-// (hi, lo) -> FP64, rounded to nearest (ties away from zero) in integer
-// arithmetic: M = hi's 24-bit significand << 29 plus lo aligned to it.
-__device__ __forceinline__ double df_to_double(dfl v) {
+// (hi, lo) * 2^-halvings -> FP64, rounded to nearest (ties away from zero) in
+// integer arithmetic: M = hi's 24-bit significand << 29 plus lo aligned to it.
+// (0 <= halvings < 512: the FP64 exponent stays above 0.)
+__device__ __forceinline__ double df_to_double(dfl v, int halvings = 0) {
   unsigned hb = (unsigned)__float_as_int(v.hi), lb = (unsigned)__float_as_int(v.lo);
   int eh = (int)((hb >> 23) & 0xffu);
   if (eh == 0) return 0.0;  // hi is zero (or FP32-subnormal): value below 2^-126
@@ -175,7 +176,7 @@ __device__ __forceinline__ double df_to_double(dfl v) {
     else L = 0;
     if ((hb ^ lb) & 0x80000000u) M -= L; else M += L;
   }
-  int E = eh + 896;  // FP64 biased exponent for M in [2^54, 2^55)
+  int E = eh + 896 - halvings;  // FP64 biased exponent for M in [2^54, 2^55)
   int drop = 2;
   if (M >= (1ll << 55)) {
     drop = 3;
@@ -212,6 +213,11 @@ struct PolF64 {
 
   __device__ static __forceinline__ R from_glob(Glob a) { return R{a.x, a.y}; }
   __device__ static __forceinline__ Glob to_glob(R r) { return make_double2(r.re, r.im); }
+  // times 2^-halvings (exact)
+  __device__ static __forceinline__ Glob to_glob_halved(R r, int halvings) {
+    const double f = __longlong_as_double((long long)(1023 - halvings) << 52);
+    return make_double2(r.re * f, r.im * f);
+  }
   __device__ static __forceinline__ R from_smem(Smem a) { return R{a.x, a.y}; }
   __device__ static __forceinline__ Smem to_smem(R r) { return make_double2(r.re, r.im); }
   __device__ static __forceinline__ Coef coef(const double* m, const float*) {
@@ -236,6 +242,11 @@ struct PolF64 {
     u.im = (a.im + b.im) * kSqHalf;
     v.re = (a.re - b.re) * kSqHalf;
     v.im = (a.im - b.im) * kSqHalf;
+  }
+  __device__ static __forceinline__ void sum_difference(R& u, R& v) {
+    R a = u, b = v;
+    u = R{a.re + b.re, a.im + b.im};
+    v = R{a.re - b.re, a.im - b.im};
   }
   __device__ static __forceinline__ void ry(R& u, R& v, const Coef& g) {
     double c = g.v[0], s = g.v[4];
@@ -277,6 +288,9 @@ struct PolDF {
   __device__ static __forceinline__ Glob to_glob(R r) {
     return make_double2(df_to_double(r.re), df_to_double(r.im));
   }
+  __device__ static __forceinline__ Glob to_glob_halved(R r, int halvings) {
+    return make_double2(df_to_double(r.re, halvings), df_to_double(r.im, halvings));
+  }
   __device__ static __forceinline__ R from_smem(Smem a) {
     return R{dfl{a.x, a.y}, dfl{a.z, a.w}};
   }
@@ -314,6 +328,11 @@ struct PolDF {
     v.re = df_mul(df_sub(a.re, b.re), s);
     v.im = df_mul(df_sub(a.im, b.im), s);
   }
+  __device__ static __forceinline__ void sum_difference(R& u, R& v) {
+    R a = u, b = v;
+    u = R{df_add(a.re, b.re), df_add(a.im, b.im)};
+    v = R{df_sub(a.re, b.re), df_sub(a.im, b.im)};
+  }
   __device__ static __forceinline__ void ry(R& u, R& v, const Coef& g) {
     dfl c = g.v[0], s = g.v[4];
     R a = u, b = v;
@@ -349,6 +368,10 @@ struct PolF32 {
 
   __device__ static __forceinline__ R from_glob(Glob a) { return R{a.x, a.y}; }
   __device__ static __forceinline__ Glob to_glob(R r) { return make_float2(r.re, r.im); }
+  __device__ static __forceinline__ Glob to_glob_halved(R r, int halvings) {
+    const float f = __int_as_float((127 - halvings) << 23);
+    return make_float2(r.re * f, r.im * f);
+  }
   __device__ static __forceinline__ R from_smem(Smem a) { return R{a.x, a.y}; }
   __device__ static __forceinline__ Smem to_smem(R r) { return make_float2(r.re, r.im); }
   __device__ static __forceinline__ Coef coef(const double*, const float* hl) {
@@ -376,6 +399,11 @@ struct PolF32 {
     u.im = mul_sq_half(a.im + b.im);
     v.re = mul_sq_half(a.re - b.re);
     v.im = mul_sq_half(a.im - b.im);
+  }
+  __device__ static __forceinline__ void sum_difference(R& u, R& v) {
+    R a = u, b = v;
+    u = R{a.re + b.re, a.im + b.im};
+    v = R{a.re - b.re, a.im - b.im};
   }
   __device__ static __forceinline__ void ry(R& u, R& v, const Coef& g) {
     float c = g.v[0], s = g.v[4];
@@ -409,6 +437,7 @@ __device__ __forceinline__ void apply_pair(int kind, typename P::R& u,
     case 3: P::cmul(v, g, 6); break;             // GK_PHASE
     case 4: P::cmul(u, g, 0); P::cmul(v, g, 6); break;  // GK_DIAG
     case 6: P::dense_r(u, v, g); break;          // GK_DENSE_R
+    case 9: P::sum_difference(u, v); break;      // GK_HU
     default: P::ry(u, v, g); break;              // GK_RY
   }
 }

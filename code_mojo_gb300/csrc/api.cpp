@@ -206,6 +206,7 @@ struct Step {
   bool digits = false;             // tensor-core pass in the complex128 digit form
   bool unitaries = false;          // tile pass: holds dense unitaries (GK_UNITARY ops)
   bool fans = false;               // tile pass: holds phase fans
+  int halvings = 0;                // tile pass: results are stored times 2^-halvings
 };
 
 // a^-1 mod N for gcd(a, N) = 1 (extended Euclid, as modinv in algos/shor.mojo:46-53)
@@ -419,7 +420,8 @@ static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opt
         size_t b0 = pg.blocks.size(), i0 = pg.images.size(), o0 = pg.offsets.size();
         // the most blocks for which the block pass is still the cheaper form
         std::vector<TileOp> merged;
-        merge_phases(ps.tile, merged, nullptr);
+        int halvings = 0;
+        merge_phases(ps.tile, merged, nullptr, &halvings);
         const double cu = cuda_core_units(merged);
         int max_blocks = 0;
         while (max_blocks < kMaxPassBlocks && (double)(max_blocks + 1) * block_units < cu) ++max_blocks;
@@ -444,7 +446,7 @@ static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opt
         s.tile = ps.tile;
         s.prog_off = prog.size();
         s.tile.ops.clear();
-        s.fans = merge_phases(ps.tile, s.tile.ops, &pg.umats) > 0;
+        s.fans = merge_phases(ps.tile, s.tile.ops, &pg.umats, &s.halvings) > 0;
         s.nprog = (int)s.tile.ops.size();
         for (const TileOp& t : s.tile.ops) s.unitaries |= t.kind == GK_UNITARY;
         prog.insert(prog.end(), s.tile.ops.begin(), s.tile.ops.end());
@@ -722,7 +724,7 @@ static void run_steps(State& st, const std::vector<Step>& steps, const Program& 
         launch_tile_pass(st, st.d_prog + s.prog_off, s.nprog, s.tile,
                          s.unitaries || s.fans ? reinterpret_cast<const double*>(st.d_aux + pg.umats_offset())
                                                : nullptr,
-                         s.unitaries, s.fans);
+                         s.unitaries, s.fans, s.halvings);
         break;
       case Step::TBLOCK:
         if (s.digits) {

@@ -41,6 +41,7 @@ struct BatchPass {
   TileGeom geo;
   uint32_t op_begin;
   uint32_t nops;
+  int32_t halvings;  // results are stored times 2^-halvings
 };
 
 struct BatchDesc {
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(kTileThreads) k_batch(const BatchDesc d) {
       if (task.kind == TASK_TILE) {
         TileGeom geo = bp.geo;
         run_tile<P, true, false, kFans>(static_cast<typename P::Glob*>(d.pool) + bp.offset, d.ops + bp.op_begin,
-                                        (int)bp.nops, geo, task.tile, smem_raw, d.fans);
+                                        (int)bp.nops, geo, task.tile, smem_raw, d.fans, bp.halvings);
       } else if constexpr (sizeof(typename P::Glob) == 8) {
         float2* base = reinterpret_cast<float2*>(d.pool) + bp.offset + ((uint64_t)task.tile << bp.geo.K);
         const int cnt = 1 << bp.geo.K;
@@ -331,7 +332,7 @@ static Batch* build_batch(int ncirc, const int32_t* nq, const bf_op* const* ops,
         bp.geo.L = ps.tile.L;
         for (int j = 0; j < ps.tile.K; ++j) bp.geo.q[j] = ps.tile.q[j];
         bp.op_begin = (uint32_t)prog.size();
-        const bool fans = merge_phases(ps.tile, prog, &fan_pool) > 0;
+        const bool fans = merge_phases(ps.tile, prog, &fan_pool, &bp.halvings) > 0;
         b->fans |= fans;
         bp.nops = (uint32_t)(prog.size() - bp.op_begin);
         circ_passes[c].push_back((uint32_t)passes.size());

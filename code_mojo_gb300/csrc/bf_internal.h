@@ -97,7 +97,8 @@ enum GKind : int32_t {
   GK_RY = 5,     // real rotation [[c,-s],[s,c]]: m[0] = c, m[4] = s
   GK_DENSE_R = 6, // full 2x2 matrix whose m00 is real (m[1] == 0), as in every U3
   GK_UNITARY = 7, // dense 2^um x 2^um matrix on qubits target .. target + um - 1
-  GK_FAN = 8      // tile ops only: a phase fan on its own (below)
+  GK_FAN = 8,     // tile ops only: a phase fan on its own (below)
+  GK_HU = 9       // tile ops only: a Hadamard without its factor, (u+v), (u-v)
 };
 
 // Dense unitaries of up to this many qubits join fused runs (tile passes
@@ -356,9 +357,10 @@ void sync_state(State& st);
 // Kernel launchers (device code lives in the .cu files).
 void launch_gate(State& s, const GateInstr& g);
 // d_pool: the device copy of the program's pool (unitary matrices and phase
-// fans); unitaries / fans: the pass holds GK_UNITARY ops / phase fans
-void launch_tile_pass(State& s, const TileOp* d_ops, int nops, const TilePass& p, const double* d_pool = nullptr,
-                      bool unitaries = false, bool fans = false);
+// fans); unitaries / fans: the pass holds GK_UNITARY ops / phase fans; the
+// results are multiplied by 2^-halvings
+void launch_tile_pass(State& s, const TileOp* d_ops, int nops, const TilePass& p, const double* d_pool, bool unitaries,
+                      bool fans, int halvings);
 void launch_block_pass(State& st, const Blk5* d_blocks, int nblocks, const unsigned char* d_images,
                        const uint16_t* d_offsets, const TilePass& p);
 // complex128 digit blocks (BLOCK_DIGITS); d_exp holds the scale exponent
@@ -438,8 +440,10 @@ double core_units(int kind, int um);
 // fans (see TileOp): each phase waits until a gate acts non-diagonally on one
 // of its qubits, and the phases that meet that gate's target are multiplied
 // into one fan before it.  Tables go to `pool` (null: the ops only, for a
-// cost estimate).  Returns the number of fans.
-int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<double>* pool);
+// cost estimate).  Hadamards go in pairs as GK_HU, whose two factors of
+// sqrt(1/2) make an exact 1/2: *halvings of them are left to the pass's store.
+// Returns the number of fans.
+int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<double>* pool, int* halvings);
 
 // bf_execute's body on a prepared state; stream, event and SM count of a
 // state; releasing every buffer a state owns (api.cpp).

@@ -259,6 +259,8 @@ static bool fan_takes(const PhaseTerm& t, uint32_t centre_loc, uint64_t centre_o
   return (l >> a) == 0 || (l & ((1u << a) - 1u)) == 0;
 }
 
+constexpr int kMaxHalvings = 12;
+
 // One table: entry x is the product of the factors whose mask is within x.
 static void fan_table(const std::vector<std::pair<uint32_t, const double*>>& terms, int bits, int shift, double* out) {
   std::vector<double> one(2 * (size_t)bits, 0.0);  // product per single-bit mask
@@ -289,7 +291,8 @@ static void fan_table(const std::vector<std::pair<uint32_t, const double*>>& ter
   }
 }
 
-int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<double>* pool) {
+int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<double>* pool, int* halvings) {
+  const size_t first = out.size();
   const int K = tp.K, a = K / 2;
   std::vector<PhaseTerm> pending;
   int fans = 0;
@@ -394,6 +397,19 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
     out.push_back(g);
   }
   flush(pending, 0u, nullptr);
+  // pairs of Hadamards without their factors: u + v and u - v take 44 of a
+  // Hadamard's 72 double-float instructions, and the exact 1/2 per pair costs
+  // the store nothing; at most kMaxHalvings, so that values grow by no more
+  // than 2^kMaxHalvings inside the pass
+  int h = 0;
+  for (size_t k = first; k < out.size(); ++k) h += out[k].kind == GK_H;
+  *halvings = std::min(h / 2, kMaxHalvings);
+  h = 2 * *halvings;
+  for (size_t k = first; k < out.size() && h > 0; ++k)
+    if (out[k].kind == GK_H) {
+      out[k].kind = GK_HU;
+      --h;
+    }
   return fans;
 }
 
@@ -498,15 +514,16 @@ static double pass_core_units(const std::vector<const GateInstr*>& remaining, ui
 }
 
 // A tile op's cost on the CUDA cores, in units of one dense gate over the
-// tile (double-float: about 134 instructions per pair, a Hadamard 86, a fan
-// 76 on its half of the amplitudes; an m-qubit unitary does 2^m complex
+// tile (double-float: about 134 instructions per pair, a Hadamard 58 without
+// its factor, a fan 76 on its half of the amplitudes; an m-qubit unitary does 2^m complex
 // products per amplitude against a dense gate's 2).
 double core_units(int kind, int um) {
   switch (kind) {
     case GK_SWAP: return 0.5;
     case GK_PHASE: return 0.4;
     case GK_DIAG: return 0.6;
-    case GK_H: return 0.65;
+    case GK_H:
+    case GK_HU: return 0.45;
     case GK_FAN: return 0.6;
     case GK_UNITARY: return (double)(1 << (um - 1));
     default: return 1.0;

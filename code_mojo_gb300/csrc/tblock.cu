@@ -1057,15 +1057,15 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_tblock_dg(const DgPassArgs a)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kDgTmemCols) : "memory");
 }
 
-// scale exponent e (scale = 2^e >= 2 * norm) from norm-squared partials
+// scale exponent e (scale = 2^e >= 2 * norm) from norm-squared partials: one
+// warp, 32 independent sums folded at the end (a single thread's chain of
+// additions took 70 us before every circuit's first digit pass)
 __global__ void k_digit_scale(const double* __restrict__ partial, int blocks, int* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double hi = 0, lo = 0;
-  for (int b = 0; b < blocks; ++b) {
-    hi += partial[2 * b];
-    lo += partial[2 * b + 1];
-  }
-  const double nrm = sqrt(hi + lo) * (1.0 + 1e-6);
+  double sum = 0;
+  for (int b = threadIdx.x; b < blocks; b += 32) sum += partial[2 * b] + partial[2 * b + 1];
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  if (threadIdx.x != 0) return;
+  const double nrm = sqrt(sum) * (1.0 + 1e-6);
   int e = 1;
   if (nrm > 0) {
     int k = 0;

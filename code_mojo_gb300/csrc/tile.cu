@@ -27,13 +27,15 @@ namespace bf {
 template <class P, bool kUnitaries, bool kFans>
 __global__ void __launch_bounds__(kTileThreads) k_tile(typename P::Glob* __restrict__ s,
                                                        const TileOp* __restrict__ ops, int nops,
-                                                       const TileGeom geo, const double* __restrict__ pool) {
+                                                       const TileGeom geo, const double* __restrict__ pool,
+                                                       int halvings) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  run_tile<P, false, kUnitaries, kFans>(s, ops, nops, geo, blockIdx.x, smem_raw, pool);
+  run_tile<P, false, kUnitaries, kFans>(s, ops, nops, geo, blockIdx.x, smem_raw, pool, halvings);
 }
 
 template <class P, bool kUnitaries, bool kFans>
-static void launch_tile_form(State& st, const TileOp* d_ops, int nops, const TileGeom& geo, const double* d_pool) {
+static void launch_tile_form(State& st, const TileOp* d_ops, int nops, const TileGeom& geo, const double* d_pool,
+                             int halvings) {
   static PerDeviceOnce configured;  // one per instantiation
   configured.run(st.device, [] {
     BF_CUDA(cudaFuncSetAttribute(k_tile<P, kUnitaries, kFans>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -43,14 +45,14 @@ static void launch_tile_form(State& st, const TileOp* d_ops, int nops, const Til
   if (blocks > 0x7fffffffull) fail(BF_EUNSUPPORTED, "tile grid too large");
   k_tile<P, kUnitaries, kFans><<<(unsigned)blocks, kTileThreads,
                                  tile_smem_bytes<P>(geo.K, geo.L, kUnitaries, kFans), st.stream>>>(
-      static_cast<typename P::Glob*>(st.amp), d_ops, nops, geo, d_pool);
+      static_cast<typename P::Glob*>(st.amp), d_ops, nops, geo, d_pool, halvings);
   BF_CUDA(cudaGetLastError());
   st.launches++;
 }
 
 template <class P>
 static void launch_tile_p(State& st, const TileOp* d_ops, int nops, const TilePass& p, const double* d_pool,
-                          bool unitaries, bool fans) {
+                          bool unitaries, bool fans, int halvings) {
   TileGeom geo;
   geo.K = p.K;
   geo.L = p.L;
@@ -58,18 +60,18 @@ static void launch_tile_p(State& st, const TileOp* d_ops, int nops, const TilePa
   for (int j = 0; j < p.K; ++j) geo.q[j] = p.q[j];
   for (int j = 0; j < geo.L; ++j)
     if (geo.q[j] != j) fail(BF_EINVAL, "internal: tile qubits must start with 0..%d", geo.L - 1);
-  if (unitaries && fans) launch_tile_form<P, true, true>(st, d_ops, nops, geo, d_pool);
-  else if (unitaries) launch_tile_form<P, true, false>(st, d_ops, nops, geo, d_pool);
-  else if (fans) launch_tile_form<P, false, true>(st, d_ops, nops, geo, d_pool);
-  else launch_tile_form<P, false, false>(st, d_ops, nops, geo, d_pool);
+  if (unitaries && fans) launch_tile_form<P, true, true>(st, d_ops, nops, geo, d_pool, halvings);
+  else if (unitaries) launch_tile_form<P, true, false>(st, d_ops, nops, geo, d_pool, halvings);
+  else if (fans) launch_tile_form<P, false, true>(st, d_ops, nops, geo, d_pool, halvings);
+  else launch_tile_form<P, false, false>(st, d_ops, nops, geo, d_pool, halvings);
 }
 
 void launch_tile_pass(State& st, const TileOp* d_ops, int nops, const TilePass& p, const double* d_pool,
-                      bool unitaries, bool fans) {
+                      bool unitaries, bool fans, int halvings) {
   switch (st.prec) {
-    case PREC_F64: launch_tile_p<PolF64>(st, d_ops, nops, p, d_pool, unitaries, fans); break;
-    case PREC_DF: launch_tile_p<PolDF>(st, d_ops, nops, p, d_pool, unitaries, fans); break;
-    default: launch_tile_p<PolF32>(st, d_ops, nops, p, d_pool, unitaries, fans); break;
+    case PREC_F64: launch_tile_p<PolF64>(st, d_ops, nops, p, d_pool, unitaries, fans, halvings); break;
+    case PREC_DF: launch_tile_p<PolDF>(st, d_ops, nops, p, d_pool, unitaries, fans, halvings); break;
+    default: launch_tile_p<PolF32>(st, d_ops, nops, p, d_pool, unitaries, fans, halvings); break;
   }
 }
 

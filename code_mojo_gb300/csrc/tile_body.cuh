@@ -54,6 +54,7 @@ __device__ __forceinline__ void tile_gate(int kind, typename P::Smem* amp, int T
   switch (kind) {
     case GK_DENSE: tile_pairs<P, GK_DENSE, kCtl>(amp, TS, tloc, cml, g); break;
     case GK_H: tile_pairs<P, GK_H, kCtl>(amp, TS, tloc, cml, g); break;
+    case GK_HU: tile_pairs<P, GK_HU, kCtl>(amp, TS, tloc, cml, g); break;
     case GK_SWAP: tile_pairs<P, GK_SWAP, kCtl>(amp, TS, tloc, cml, g); break;
     case GK_PHASE: tile_pairs<P, GK_PHASE, kCtl>(amp, TS, tloc, cml, g); break;
     case GK_DIAG: tile_pairs<P, GK_DIAG, kCtl>(amp, TS, tloc, cml, g); break;
@@ -212,10 +213,11 @@ __host__ __device__ inline size_t tile_fan_bytes(int K) {
 // `smem_raw` also holds the staged matrix.
 // kFans: the ops may carry phase fans; pool then holds their tables and
 // constants, and `smem_raw` also holds the staged ones (tile_smem_bytes).
+// The results are stored times 2^-halvings.
 template <class P, bool kL2Loads = false, bool kUnitaries = false, bool kFans = false>
 __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const TileOp* __restrict__ ops, int nops,
                                          const TileGeom& geo, uint64_t tile, unsigned char* smem_raw,
-                                         const double* __restrict__ pool = nullptr) {
+                                         const double* __restrict__ pool, int halvings) {
   using R = typename P::R;
   using S = typename P::Smem;
   const int K = geo.K, L = geo.L;
@@ -355,6 +357,7 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
         switch (kind) {
           case GK_FAN: tile_pairs_fan<P, GK_FAN>(amp, TS, tloc, g, f); break;
           case GK_H: tile_pairs_fan<P, GK_H>(amp, TS, tloc, g, f); break;
+          case GK_HU: tile_pairs_fan<P, GK_HU>(amp, TS, tloc, g, f); break;
           case GK_DENSE_R: tile_pairs_fan<P, GK_DENSE_R>(amp, TS, tloc, g, f); break;
           case GK_RY: tile_pairs_fan<P, GK_RY>(amp, TS, tloc, g, f); break;
           default: tile_pairs_fan<P, GK_DENSE>(amp, TS, tloc, g, f); break;
@@ -381,7 +384,7 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
 
   for (int e = tid; e < TS; e += kTileThreads) {
     uint64_t gi = obase | (uint64_t)(e & lowmask) | hoff[e >> L];
-    s[gi] = P::to_glob(P::from_smem(amp[e]));
+    s[gi] = P::to_glob_halved(P::from_smem(amp[e]), halvings);
   }
 }
 

@@ -4,6 +4,7 @@
 // constants as the kernel reads them.
 //   fan_model <ops file> <state in> <state out> <tile qubits> <block units>
 // Prints: tile passes, gate steps, fans, phases left as ops of their own.
+#include <cmath>
 #include <complex>
 #include <cstdio>
 #include <cstdlib>
@@ -86,7 +87,8 @@ int main(int argc, char** argv) {
     ++tiles;
     const TilePass& tp = ps.tile;
     std::vector<TileOp> merged;
-    const int made = merge_phases(tp, merged, &g_pool);
+    int halvings = 0, bare = 0;
+    const int made = merge_phases(tp, merged, &g_pool, &halvings);
     fans += made;
     uint64_t tile_bits = 0;
     for (int j = 0; j < tp.K; ++j) tile_bits |= 1ull << tp.q[j];
@@ -121,7 +123,11 @@ int main(int argc, char** argv) {
         }
         if (t.kind == GK_FAN) continue;
       }
-      if (t.kind == GK_UNITARY) {
+      if (t.kind == GK_HU) {
+        const double m[8] = {1, 0, 1, 0, 1, 0, -1, 0};
+        gate(s, tp.q[t.tloc], cm, m);
+        ++bare;
+      } else if (t.kind == GK_UNITARY) {
         unitary(s, tp.q[t.tloc], t.um, cm, g_pool.data() + t.uoff);
       } else if (t.tloc >= 0) {
         gate(s, tp.q[t.tloc], cm, t.m);
@@ -130,6 +136,8 @@ int main(int argc, char** argv) {
           if ((i & cm) == cm) s[i] *= ((i >> t.tglob) & 1) ? cd(t.m[6], t.m[7]) : cd(t.m[0], t.m[1]);
       }
     }
+    if (bare != 2 * halvings) return 9;
+    for (cd& x : s) x *= std::ldexp(1.0, -halvings);
   }
   std::ofstream fw(argv[3], std::ios::binary);
   fw.write(reinterpret_cast<const char*>(s.data()), (std::streamsize)(s.size() * sizeof(cd)));
