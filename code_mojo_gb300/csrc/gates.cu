@@ -27,11 +27,13 @@ struct GateArgs {
 // Each thread takes gate_unroll pair bases a grid-stride apart and issues
 // all their loads before any arithmetic, so that enough bytes are in flight
 // to keep HBM busy (a state far larger than L2 is read once: streaming loads
-// and stores).  Measured at 30 qubits: the arithmetic kinds at complex128
-// keep two (more registers cut occupancy), the data-movement kinds eight.
+// and stores).  At complex128 the arithmetic kinds keep two (more registers
+// cut occupancy) and the data-movement kinds four: a P at 26 qubits takes 215
+// us with four and 233 with eight, a CX at 20 qubits 6.2 and 8.7, at 24 41.9
+// and 43.9, at 28 648 and 640.  At complex64 they keep four and eight.
 template <class P, int KIND>
 __host__ __device__ constexpr int gate_unroll() {
-  return (KIND == GK_SWAP || KIND == GK_PHASE) ? 8 : (sizeof(typename P::Glob) == 16 ? 2 : 4);
+  return (sizeof(typename P::Glob) == 16 ? 2 : 4) * ((KIND == GK_SWAP || KIND == GK_PHASE) ? 2 : 1);
 }
 
 template <class P, int KIND>
