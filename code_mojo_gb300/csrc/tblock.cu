@@ -399,19 +399,27 @@ static_assert(kDgCols == 8 && kDgLoadIters * 2 == kBlockTableEntries / kDgThread
 // issue order; the first group to reach a level initialises it.  Six
 // digits: the 26 pairs with i + j <= 6.  Five digits: the 20 pairs with
 // i <= 4, j <= 5, i + j <= 5.
+//
+// They are issued in two stages, the lower levels (5 to 2, or 6 to 3) first,
+// with a barrier each: the epilogue takes the levels from the lowest up and
+// starts on the first stage's under the MMAs of the second.  Digit planes are
+// written back only when no stage still to run reads them: under the second
+// stage, which reads planes 0 and 1 (0 to 2), the epilogue writes planes 4 and
+// 3 (5 and 4).  130.3 against 132.6 ms for the 23 passes of a 28-qubit layered
+// circuit.  Three stages of two levels overlap more but need MMAs of N = 128,
+// which take nearly as long as those of N = 256: 155 ms.
 struct DgGroup {
   int i, j0, nj, init;
 };
-#define BF_DG_GROUPS6                                                                                 \
-  {                                                                                                   \
-    {0, 0, 4, 1}, {0, 4, 2, 1}, /* levels 0..5 first written */                                       \
-        {1, 5, 1, 1},           /* level 6 first written */                                           \
-        {1, 0, 4, 0}, {1, 4, 1, 0}, {2, 0, 4, 0}, {2, 4, 1, 0}, {3, 0, 4, 0}, {4, 0, 3, 0}, {5, 0, 2, 0} \
+#define BF_DG_GROUPS6                                                                                    \
+  {                                                                                                      \
+    {1, 2, 4, 1}, {2, 1, 4, 0}, {3, 0, 4, 0}, {0, 3, 3, 0}, {4, 0, 3, 0}, {5, 0, 2, 0}, /* levels 6..3 */ \
+        {0, 0, 3, 1}, {1, 0, 2, 0}, {2, 0, 1, 0}                                        /* levels 2..0 */ \
   }
-#define BF_DG_GROUPS5                                                                                 \
-  {                                                                                                   \
-    {0, 0, 4, 1}, {0, 4, 2, 1}, /* levels 0..5 first written */                                       \
-        {1, 0, 4, 0}, {1, 4, 1, 0}, {2, 0, 4, 0}, {3, 0, 3, 0}, {4, 0, 2, 0}                          \
+#define BF_DG_GROUPS5                                                                                    \
+  {                                                                                                      \
+    {0, 2, 4, 1}, {1, 1, 4, 0}, {2, 0, 4, 0}, {3, 0, 3, 0}, {4, 0, 2, 0}, /* levels 5..2 */              \
+        {0, 0, 2, 1}, {1, 0, 1, 0}                                        /* levels 1, 0 */              \
   }
 
 // 8 columns of the thread's TMEM lane
@@ -650,7 +658,7 @@ __device__ __forceinline__ uint32_t sq_bound_units_fixed(long long V) {
 template <int D>
 __device__ __forceinline__ DgGroup dg_group(int gi) {
   if constexpr (D == 6) {
-    constexpr DgGroup g[10] = BF_DG_GROUPS6;
+    constexpr DgGroup g[9] = BF_DG_GROUPS6;
     return g[gi];
   } else {
     constexpr DgGroup g[7] = BF_DG_GROUPS5;
@@ -658,7 +666,10 @@ __device__ __forceinline__ DgGroup dg_group(int gi) {
   }
 }
 template <int D>
-constexpr int kDgGroupCount = D == 6 ? 10 : 7;
+constexpr int kDgGroupCount = D == 6 ? 9 : 7;
+// the groups of the first stage
+template <int D>
+constexpr int kDgFirstStage = D == 6 ? 6 : 5;
 
 // The CTA's pipeline state, carried from tile to tile.  Block k of the CTA
 // (counting every tile's blocks) uses image buffer k & 1, whose barrier is
@@ -744,7 +755,10 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
     if (dg_wait_image(f, a, p, p.kimg)) {
       const uint32_t sBk = f.sB + (p.kimg & 1u) * kDigitImageBytes;
 #pragma unroll
-      for (int gi = 0; gi < kDgGroupCount<D>; ++gi) dg_mma_group(f, sBk, dg_group<D>(gi));
+      for (int gi = 0; gi < kDgGroupCount<D>; ++gi) {
+        dg_mma_group(f, sBk, dg_group<D>(gi));
+        if (gi + 1 == kDgFirstStage<D>) mma_commit(f.bar_mma + 8u);
+      }
       dg_commit(f, a, p, p.kimg, 0, obase, has_next);
     } else {
       issue_lost = true;
@@ -756,8 +770,13 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
     const uint32_t sBn = f.sB + ((k + 1) & 1u) * kDigitImageBytes;
     const uint2 dest = my_dests4(a.offsets, f.blk[bi].offs);
     bool lost = issue_lost;     // no MMAs were issued: the wait below expires too
-    if (!mbar_wait(f.bar_mma, k & 1u, a.spin_limit)) lost = true;
-    tc_fence_after();
+    // the first stage's levels, then (from level 1 or 2 down) the others
+    auto stage = [&](int s) {
+      if (s == D || s == D - 4) {
+        if (!lost && !mbar_wait(f.bar_mma + (s == D ? 8u : 0u), k & 1u, a.spin_limit)) lost = true;
+        tc_fence_after();
+      }
+    };
     // Level s holds digit position s + 1 of the result.  From the lowest
     // level up: t = sum + carry, digit = t - 256 round(t / 256), carry the
     // rest; positions D and D + 1 only round; position 0 is the last carry.
@@ -782,6 +801,7 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
 #pragma unroll
       for (int s = D; s >= 1; s -= 2) {
         float d0[kDgCols], d1[kDgCols];
+        stage(s);
         tmem_ld8x2(f.tlane + 64u * (uint32_t)s, f.tlane + 64u * (uint32_t)(s - 1), d0, d1);
         level(s, d0);
         level(s - 1, d1);
@@ -824,6 +844,7 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
 #pragma unroll
       for (int s = D; s >= 1; s -= 2) {
         float d0[kDgCols], d1[kDgCols];
+        stage(s);
         tmem_ld8x2(f.tlane + 64u * (uint32_t)s, f.tlane + 64u * (uint32_t)(s - 1), d0, d1);
         level(s, d0);
         level(s - 1, d1);
@@ -860,7 +881,10 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
       tc_fence_after();
       if (dg_wait_image(f, a, p, k + 1)) {
 #pragma unroll
-        for (int gi = 0; gi < kDgGroupCount<D>; ++gi) dg_mma_group(f, sBn, dg_group<D>(gi));
+        for (int gi = 0; gi < kDgGroupCount<D>; ++gi) {
+          dg_mma_group(f, sBn, dg_group<D>(gi));
+          if (gi + 1 == kDgFirstStage<D>) mma_commit(f.bar_mma + 8u);
+        }
         dg_commit(f, a, p, k + 1, bi + 1, obase, has_next);
       } else {
         issue_lost = true;
@@ -877,7 +901,8 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_tblock_dg(const DgPassArgs a)
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kDgSmemBar);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kDgSmemBar + 72);
   Blk5* blk = reinterpret_cast<Blk5*>(sm + kDgSmemBlk);
-  // bars[0], bars[1]: image buffers; bars[2]: the MMAs of a block
+  // bars[0], bars[1]: image buffers; bars[2]: the MMAs of a block; bars[3]:
+  // those of its first stage
   const uint32_t bar_b = smem_u32(&bars[0]), bar_mma = smem_u32(&bars[2]);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -891,6 +916,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_tblock_dg(const DgPassArgs a)
     mbar_init(bar_b, 1);
     mbar_init(bar_b + 8u, 1);
     mbar_init(bar_mma, 1);
+    mbar_init(bar_mma + 8u, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int h = tid; h < 128; h += kDgThreads) {
