@@ -149,7 +149,9 @@ struct TileOp {
   uint64_t cmask_out; // control bits outside the tile (global positions)
   double m[8];
   float mhl[16];
-  int32_t um;         // GK_UNITARY: qubit count; 0 otherwise
+  int32_t um;         // GK_UNITARY: qubit count; in an op with a fan, a
+                      // Hadamard of the same target that goes before the fan
+                      // (GK_H or GK_HU, 0: none)
   int32_t uoff;       // GK_UNITARY: offset (in doubles) of its matrix in the
                       // program's pool
   // The phase fan applied before the op (alone for GK_FAN): the product of

@@ -296,6 +296,7 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
   const int K = tp.K, a = K / 2;
   std::vector<PhaseTerm> pending;
   int fans = 0;
+  std::vector<uint32_t> fan_bits(1, 0u);  // by fan: the tile bits of its phases
   // fills op's fan from the terms around one centre
   auto make_fan = [&](TileOp& op, const std::vector<PhaseTerm>& terms, uint32_t centre_loc) {
     std::vector<std::pair<uint32_t, const double*>> ta, tb;
@@ -307,6 +308,8 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
       else tb.emplace_back(l, t.op->m + 6);
     }
     op.fan = ++fans;
+    fan_bits.push_back(0u);
+    for (const PhaseTerm& t : terms) fan_bits.back() |= t.loc;
     op.fan_shape = a | (ta.empty() ? 0 : kFanA) | (tb.empty() ? 0 : kFanB);
     op.fan_consts = (int32_t)consts.size();
     if (!pool) return;
@@ -330,7 +333,7 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
   // can join; true when one did.
   auto flush = [&](std::vector<PhaseTerm> terms, uint32_t centre, TileOp* gate) {
     bool joined = false;
-    while ((int)terms.size() >= kMinFanTerms && fans < kMaxPassFans && (!pool || pool->size() < kMaxFanPool)) {
+    while (!terms.empty() && fans < kMaxPassFans && (!pool || pool->size() < kMaxFanPool)) {
       uint32_t cl = centre;
       uint64_t co = 0;
       if (!centre) {
@@ -353,7 +356,9 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
         if (((t.loc & cl) || (t.out & co)) && fan_takes(t, cl, co, a)) in.push_back(t);
         else rest.push_back(t);
       }
-      if ((int)in.size() < kMinFanTerms) break;
+      // one phase of the target alone costs a gate in hand one product
+      const bool lone = gate && centre && in.size() == 1 && (in[0].loc & ~cl) == 0;
+      if ((int)in.size() < kMinFanTerms && !lone) break;
       if (gate && centre) {
         make_fan(*gate, in, cl);
         joined = true;
@@ -397,19 +402,41 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
     out.push_back(g);
   }
   flush(pending, 0u, nullptr);
+  // A Hadamard goes into the next op on its target where that has a fan and
+  // nothing between them touches the target: the pair is read and written once.
+  auto touches = [&](const TileOp& op) {
+    uint32_t m = op.cmask_loc | fan_bits[(size_t)op.fan];
+    if (op.kind == GK_UNITARY) m |= ((1u << op.um) - 1u) << op.tloc;
+    else if (op.tloc >= 0) m |= 1u << op.tloc;
+    return m;
+  };
+  for (size_t k = first; k < out.size(); ++k) {
+    if (!out[k].fan || out[k].kind == GK_FAN) continue;
+    const uint32_t t = 1u << out[k].tloc;
+    size_t j = k;
+    while (j > first && !(touches(out[j - 1]) & t)) --j;
+    if (j == first) continue;
+    const TileOp& h = out[j - 1];
+    if (h.kind != GK_H || h.fan || h.tloc != out[k].tloc || h.cmask_loc || h.cmask_out) continue;
+    out[k].um = GK_H;
+    out.erase(out.begin() + (std::ptrdiff_t)(j - 1));
+    --k;
+  }
   // pairs of Hadamards without their factors: u + v and u - v take 44 of a
   // Hadamard's 72 double-float instructions, and the exact 1/2 per pair costs
   // the store nothing; at most kMaxHalvings, so that values grow by no more
   // than 2^kMaxHalvings inside the pass
+  auto is_h = [](const TileOp& op, bool before) {
+    return before ? op.kind != GK_UNITARY && op.um == GK_H : op.kind == GK_H;
+  };
   int h = 0;
-  for (size_t k = first; k < out.size(); ++k) h += out[k].kind == GK_H;
+  for (size_t k = first; k < out.size(); ++k) h += is_h(out[k], true) + is_h(out[k], false);
   *halvings = std::min(h / 2, kMaxHalvings);
   h = 2 * *halvings;
-  for (size_t k = first; k < out.size() && h > 0; ++k)
-    if (out[k].kind == GK_H) {
-      out[k].kind = GK_HU;
-      --h;
-    }
+  for (size_t k = first; k < out.size(); ++k) {
+    if (is_h(out[k], true) && h > 0 && h--) out[k].um = GK_HU;
+    if (is_h(out[k], false) && h > 0 && h--) out[k].kind = GK_HU;
+  }
   return fans;
 }
 

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstring>
+#include <type_traits>
 
 #include "amp_math.cuh"
 #include "bf_internal.h"
@@ -101,23 +102,149 @@ __device__ __forceinline__ typename P::R fan_apply(const FanView<P>& f, typename
 }
 
 // One uncontrolled in-tile gate with a fan on its target: the fan multiplies
-// the pair's second amplitude on its way into the gate (GK_FAN: alone).
+// the pair's second amplitude on its way into the gate (GK_FAN: alone),
+// after the Hadamard `before` (0: none).  With the first-layer Hadamards of a
+// 24-qubit value encoding taken along like this its passes take 1.64 against
+// 1.97 ms.
 template <class P, int KIND>
-__device__ __forceinline__ void tile_pairs_fan(typename P::Smem* amp, int TS, int tloc, const typename P::Coef& g,
-                                               const FanView<P>& f) {
+__device__ __forceinline__ void tile_pairs_fan(typename P::Smem* amp, int TS, int tloc, int before,
+                                               const typename P::Coef& g, const FanView<P>& f) {
   using R = typename P::R;
   const uint32_t low = (1u << tloc) - 1u, tb = 1u << tloc;
 #pragma unroll 1
   for (int p = threadIdx.x; p < (TS >> 1); p += kTileThreads) {
     const uint32_t i0 = (((uint32_t)p & ~low) << 1) | ((uint32_t)p & low);
     const uint32_t i1 = i0 | tb;
-    R v = fan_apply<P>(f, P::from_smem(amp[i1]), i1);
-    if (KIND != GK_FAN) {
-      R u = P::from_smem(amp[i0]);
-      apply_pair<P>(KIND, u, v, g);
-      amp[i0] = P::to_smem(u);
+    R v = P::from_smem(amp[i1]);
+    if (KIND == GK_FAN) {
+      amp[i1] = P::to_smem(fan_apply<P>(f, v, i1));
+      continue;
     }
+    R u = P::from_smem(amp[i0]);
+    if (before == GK_HU) P::sum_difference(u, v);
+    else if (before == GK_H) P::hadamard(u, v);
+    v = fan_apply<P>(f, v, i1);
+    apply_pair<P>(KIND, u, v, g);
+    amp[i0] = P::to_smem(u);
     amp[i1] = P::to_smem(v);
+  }
+}
+
+// ---- complex64: two amplitudes at a time ---------------------------------------
+// An FP32 gate is a few instructions per pair, so what a pass costs is the
+// shared-memory and index instructions around them: each thread takes the
+// amplitudes 2k and 2k + 1 as one 16-byte word (two pairs that differ in
+// local bit 0, or for a target on bit 0 one pair).  The passes of a 27-qubit
+// value encoding take 4.74 against 6.66 ms, of six layers of U3 and CX at 24
+// qubits 2.17 against 2.33.
+struct Pair32 {
+  PolF32::R a, b;  // local bit 0 = 0, 1
+};
+__device__ __forceinline__ Pair32 pair32(float4 w) { return Pair32{PolF32::R{w.x, w.y}, PolF32::R{w.z, w.w}}; }
+__device__ __forceinline__ float4 word32(const Pair32& p) { return make_float4(p.a.re, p.a.im, p.b.re, p.b.im); }
+
+// the fan on amplitudes i and i + 1 (i even)
+__device__ __forceinline__ void fan_apply2(const FanView<PolF32>& f, Pair32& v, uint32_t i) {
+  if (f.use_a) {
+    const Pair32 w = pair32(*reinterpret_cast<const float4*>(f.A + (i & f.amask)));
+    v.a = cmul_r<PolF32>(v.a, w.a);
+    v.b = cmul_r<PolF32>(v.b, w.b);
+  }
+  if (f.use_b) {
+    const PolF32::R w = PolF32::from_smem(f.B[i >> f.abits]);
+    v.a = cmul_r<PolF32>(v.a, w);
+    v.b = cmul_r<PolF32>(v.b, w);
+  }
+  if (!f.use_a && !f.use_b) {
+    v.a = cmul_r<PolF32>(v.a, f.c);
+    v.b = cmul_r<PolF32>(v.b, f.c);
+  }
+}
+
+template <int KIND>
+__device__ __forceinline__ void pair_op32(PolF32::R& u, PolF32::R& v, const PolF32::Coef& g) {
+  if (KIND == GK_SWAP) {
+    const PolF32::R t = u;
+    u = v;
+    v = t;
+  } else if (KIND != GK_FAN) {
+    apply_pair<PolF32>(KIND, u, v, g);
+  }
+}
+
+// kCtl: controls inside the tile; kFan: a fan on the target, after the
+// Hadamard `before` (such ops have no controls)
+template <int KIND, bool kCtl, bool kFan>
+__device__ __forceinline__ void tile_words(float2* amp, int TS, int tloc, uint32_t cml, const PolF32::Coef& g,
+                                           int before, const FanView<PolF32>& f) {
+  using P = PolF32;
+  float4* amp4 = reinterpret_cast<float4*>(amp);
+  if (tloc == 0) {
+#pragma unroll 2
+    for (int k = threadIdx.x; k < (TS >> 1); k += kTileThreads) {
+      if (kCtl && ((uint32_t)(2 * k) & cml) != cml) continue;
+      Pair32 p = pair32(amp4[k]);
+      if (kFan) {
+        if (before == GK_HU) P::sum_difference(p.a, p.b);
+        else if (before == GK_H) P::hadamard(p.a, p.b);
+        const uint32_t i = 2 * (uint32_t)k + 1;
+        if (f.use_a) p.b = cmul_r<P>(p.b, P::from_smem(f.A[i & f.amask]));
+        if (f.use_b) p.b = cmul_r<P>(p.b, P::from_smem(f.B[i >> f.abits]));
+        if (!f.use_a && !f.use_b) p.b = cmul_r<P>(p.b, f.c);
+      }
+      pair_op32<KIND>(p.a, p.b, g);
+      amp4[k] = word32(p);
+    }
+    return;
+  }
+  const uint32_t low = (1u << (tloc - 1)) - 1u, tb = 1u << (tloc - 1);
+  const uint32_t need = cml >> 1;
+  const bool odd_only = kCtl && (cml & 1u);
+#pragma unroll 2
+  for (uint32_t q = threadIdx.x; q < (uint32_t)(TS >> 2); q += kTileThreads) {
+    const uint32_t w0 = ((q & ~low) << 1) | (q & low), w1 = w0 | tb;
+    if (kCtl && (w0 & need) != need) continue;
+    Pair32 v = pair32(amp4[w1]);
+    if (KIND == GK_PHASE || KIND == GK_FAN) {  // the target's 1 half alone
+      if (kFan) {
+        fan_apply2(f, v, 2 * w1);
+      } else {
+        if (!odd_only) P::cmul(v.a, g, 6);
+        P::cmul(v.b, g, 6);
+      }
+      amp4[w1] = word32(v);
+      continue;
+    }
+    Pair32 u = pair32(amp4[w0]);
+    if (kFan) {
+      if (before == GK_HU) {
+        P::sum_difference(u.a, v.a);
+        P::sum_difference(u.b, v.b);
+      } else if (before == GK_H) {
+        P::hadamard(u.a, v.a);
+        P::hadamard(u.b, v.b);
+      }
+      fan_apply2(f, v, 2 * w1);
+    }
+    if (!odd_only) pair_op32<KIND>(u.a, v.a, g);
+    pair_op32<KIND>(u.b, v.b, g);
+    amp4[w0] = word32(u);
+    amp4[w1] = word32(v);
+  }
+}
+
+template <bool kCtl, bool kFan>
+__device__ __forceinline__ void tile_words_of(int kind, float2* amp, int TS, int tloc, uint32_t cml,
+                                              const PolF32::Coef& g, int before, const FanView<PolF32>& f) {
+  switch (kind) {
+    case GK_H: tile_words<GK_H, kCtl, kFan>(amp, TS, tloc, cml, g, before, f); break;
+    case GK_HU: tile_words<GK_HU, kCtl, kFan>(amp, TS, tloc, cml, g, before, f); break;
+    case GK_SWAP: tile_words<GK_SWAP, kCtl, kFan>(amp, TS, tloc, cml, g, before, f); break;
+    case GK_PHASE: tile_words<GK_PHASE, kCtl, kFan>(amp, TS, tloc, cml, g, before, f); break;
+    case GK_DIAG: tile_words<GK_DIAG, kCtl, kFan>(amp, TS, tloc, cml, g, before, f); break;
+    case GK_RY: tile_words<GK_RY, kCtl, kFan>(amp, TS, tloc, cml, g, before, f); break;
+    case GK_FAN: tile_words<GK_FAN, kCtl, kFan>(amp, TS, tloc, cml, g, before, f); break;
+    default: tile_words<GK_DENSE, kCtl, kFan>(amp, TS, tloc, cml, g, before, f); break;
   }
 }
 
@@ -279,9 +406,19 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
   }
 
   const int lowmask = (1 << L) - 1;
-  for (int e = tid; e < TS; e += kTileThreads) {
-    uint64_t gi = obase | (uint64_t)(e & lowmask) | hoff[e >> L];
-    amp[e] = P::to_smem(P::from_glob(kL2Loads ? __ldcg(s + gi) : s[gi]));
+  // complex64: two amplitudes per access where qubit 0 is a tile qubit
+  const bool words = std::is_same<P, PolF32>::value && L > 0;
+  if (words) {
+    for (int k = tid; k < (TS >> 1); k += kTileThreads) {
+      const uint64_t gi = obase | (uint64_t)((2 * k) & lowmask) | hoff[(2 * k) >> L];
+      const float4* p = reinterpret_cast<const float4*>(s + gi);
+      reinterpret_cast<float4*>(amp)[k] = kL2Loads ? __ldcg(p) : *p;
+    }
+  } else {
+    for (int e = tid; e < TS; e += kTileThreads) {
+      uint64_t gi = obase | (uint64_t)(e & lowmask) | hoff[e >> L];
+      amp[e] = P::to_smem(P::from_glob(kL2Loads ? __ldcg(s + gi) : s[gi]));
+    }
   }
   __syncthreads();
 
@@ -353,19 +490,28 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
       }
       if (tloc < 0) {  // the centre is outside the tile (and set): every amplitude
         for (int e = tid; e < TS; e += kTileThreads) amp[e] = P::to_smem(fan_apply<P>(f, P::from_smem(amp[e]), e));
+      } else if constexpr (std::is_same<P, PolF32>::value) {
+        tile_words_of<false, true>(kind, amp, TS, tloc, 0u, g, __ldg(&op->um), f);
       } else {
+        const int before = __ldg(&op->um);
         switch (kind) {
-          case GK_FAN: tile_pairs_fan<P, GK_FAN>(amp, TS, tloc, g, f); break;
-          case GK_H: tile_pairs_fan<P, GK_H>(amp, TS, tloc, g, f); break;
-          case GK_HU: tile_pairs_fan<P, GK_HU>(amp, TS, tloc, g, f); break;
-          case GK_DENSE_R: tile_pairs_fan<P, GK_DENSE_R>(amp, TS, tloc, g, f); break;
-          case GK_RY: tile_pairs_fan<P, GK_RY>(amp, TS, tloc, g, f); break;
-          default: tile_pairs_fan<P, GK_DENSE>(amp, TS, tloc, g, f); break;
+          case GK_FAN: tile_pairs_fan<P, GK_FAN>(amp, TS, tloc, before, g, f); break;
+          case GK_H: tile_pairs_fan<P, GK_H>(amp, TS, tloc, before, g, f); break;
+          case GK_HU: tile_pairs_fan<P, GK_HU>(amp, TS, tloc, before, g, f); break;
+          case GK_DENSE_R: tile_pairs_fan<P, GK_DENSE_R>(amp, TS, tloc, before, g, f); break;
+          case GK_RY: tile_pairs_fan<P, GK_RY>(amp, TS, tloc, before, g, f); break;
+          default: tile_pairs_fan<P, GK_DENSE>(amp, TS, tloc, before, g, f); break;
         }
       }
     } else if (tloc >= 0) {
-      if (cml) tile_gate<P, true>(kind, amp, TS, tloc, cml, g);
-      else tile_gate<P, false>(kind, amp, TS, tloc, 0u, g);
+      if constexpr (std::is_same<P, PolF32>::value) {
+        const FanView<P> none{};
+        if (cml) tile_words_of<true, false>(kind, amp, TS, tloc, cml, g, 0, none);
+        else tile_words_of<false, false>(kind, amp, TS, tloc, 0u, g, 0, none);
+      } else {
+        if (cml) tile_gate<P, true>(kind, amp, TS, tloc, cml, g);
+        else tile_gate<P, false>(kind, amp, TS, tloc, 0u, g);
+      }
     } else {
       // diagonal gate, target outside the tile: one entry for the whole CTA
       const int tg = __ldg(&op->tglob);
@@ -382,6 +528,15 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
     __syncthreads();
   }
 
+  if (words) {
+    const float f = __int_as_float((127 - halvings) << 23);
+    for (int k = tid; k < (TS >> 1); k += kTileThreads) {
+      const uint64_t gi = obase | (uint64_t)((2 * k) & lowmask) | hoff[(2 * k) >> L];
+      const float4 w = reinterpret_cast<const float4*>(amp)[k];
+      *reinterpret_cast<float4*>(s + gi) = make_float4(w.x * f, w.y * f, w.z * f, w.w * f);
+    }
+    return;
+  }
   for (int e = tid; e < TS; e += kTileThreads) {
     uint64_t gi = obase | (uint64_t)(e & lowmask) | hoff[e >> L];
     s[gi] = P::to_glob_halved(P::from_smem(amp[e]), halvings);

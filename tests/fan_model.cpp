@@ -105,6 +105,12 @@ int main(int argc, char** argv) {
         const double* d = g_pool.data() + t.fan_off;
         const double* c = d + 2 * (na + nb);
         if (c[4 * t.fan_consts] != 1.0 || c[4 * t.fan_consts + 1] != 0.0) return 7;
+        if (t.kind != GK_FAN && t.um) {  // the Hadamard before the fan
+          const double r = t.um == GK_HU ? 1.0 : std::sqrt(0.5);
+          const double m[8] = {r, 0, r, 0, r, 0, -r, 0};
+          gate(s, tp.q[t.tloc], 0, m);
+          bare += t.um == GK_HU;
+        }
         for (uint64_t i = 0; i < s.size(); ++i) {
           if ((i & t.cmask_out) != t.cmask_out) continue;
           uint32_t x = 0;
