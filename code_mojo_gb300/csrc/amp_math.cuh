@@ -107,6 +107,15 @@ __device__ __forceinline__ dfl df_dot3(dfl a0, dfl b0, dfl a1, dfl b1, dfl a2, d
   return df_norm(s, err);
 }
 
+// a^2 + b^2 of two FP32 values: df_dot2 without its low parts
+__device__ __forceinline__ dfl df_squares(float a, float b) {
+  const float p0 = __fmul_rn(a, a), e0 = fmaf(a, a, -p0);
+  const float p1 = __fmul_rn(b, b), e1 = fmaf(b, b, -p1);
+  float s, t;
+  two_sum(p0, p1, s, t);
+  return df_norm(s, __fadd_rn(__fadd_rn(e0, e1), t));
+}
+
 // a0*b0 + a1*b1
 __device__ __forceinline__ dfl df_dot2(dfl a0, dfl b0, dfl a1, dfl b1) {
   float p0 = __fmul_rn(a0.hi, b0.hi), e0 = fmaf(a0.hi, b0.hi, -p0);
@@ -418,10 +427,15 @@ struct PolF32 {
     v.re = mul_sq_half(a.re - b.re);
     v.im = mul_sq_half(a.im - b.im);
   }
+  // both parts in one packed instruction each (the same roundings)
   __device__ static __forceinline__ void sum_difference(R& u, R& v) {
-    R a = u, b = v;
-    u = R{a.re + b.re, a.im + b.im};
-    v = R{a.re - b.re, a.im - b.im};
+    unsigned long long a, b, s, d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(u.re), "f"(u.im));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(v.re), "f"(v.im));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(s) : "l"(a), "l"(b));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(u.re), "=f"(u.im) : "l"(s));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.re), "=f"(v.im) : "l"(d));
   }
   __device__ static __forceinline__ void ry(R& u, R& v, const Coef& g) {
     float c = g.v[0], s = g.v[4];

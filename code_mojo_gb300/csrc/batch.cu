@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kTileThreads) k_batch(const BatchDesc d) {
           dfl acc{0.f, 0.f};
           for (int e = threadIdx.x; e < cnt; e += kTileThreads) {
             float2 v = __ldcg(base + e);
-            acc = df_add(acc, df_dot2(dfl{v.x, 0.f}, dfl{v.x, 0.f}, dfl{v.y, 0.f}, dfl{v.y, 0.f}));
+            acc = df_add(acc, df_squares(v.x, v.y));
           }
           double* red = reinterpret_cast<double*>(smem_raw);
           red[threadIdx.x] = (double)acc.hi + (double)acc.lo;

@@ -70,8 +70,7 @@ __device__ __forceinline__ dfl prob_df<double2>(double2 a) {
 }
 template <>
 __device__ __forceinline__ dfl prob_df<float2>(float2 a) {
-  dfl r{a.x, 0.f}, i{a.y, 0.f};
-  return df_dot2(r, r, i, i);
+  return df_squares(a.x, a.y);
 }
 
 // the bits of x spread over the set positions of mask, ascending

@@ -24,8 +24,17 @@ namespace bf {
 // kUnitaries: the pass holds dense unitaries; kFans: phase fans (separate
 // forms, so that passes without them keep the gate loop's small register
 // count and shared memory)
+//
+// A complex64 12-qubit tile leaves room for six CTAs per SM, and six of them
+// hide the per-op latencies better than the five that 46 registers allow: the
+// passes of a 27-qubit value encoding take 4.37 against 4.74 ms (7 or 8: 4.57).
+// (0: unspecified; complex128 loses with more registers than the compiler
+// takes by itself.)
+template <class P, bool kUnitaries>
+constexpr int kTileCtas = sizeof(typename P::Glob) == 8 && !kUnitaries ? 6 : 0;
+
 template <class P, bool kUnitaries, bool kFans>
-__global__ void __launch_bounds__(kTileThreads) k_tile(typename P::Glob* __restrict__ s,
+__global__ void __launch_bounds__(kTileThreads, (kTileCtas<P, kUnitaries>)) k_tile(typename P::Glob* __restrict__ s,
                                                        const TileOp* __restrict__ ops, int nops,
                                                        const TileGeom geo, const double* __restrict__ pool,
                                                        int halvings) {
