@@ -400,9 +400,9 @@ __global__ void __launch_bounds__(kBlkThreads, 2) k_tblock(const BlkPassArgs a) 
 // of 26) with the same unit, so the five- and six-digit forms hold the same
 // integers and give the same bits.  The norm test is an exact integer bound
 // per warp (sq_bound_units), decided at the barrier that follows the
-// conversion: a tile that fails it is converted again in six digits.  On
-// the 30-qubit circuit a tile holds about 2^-9 of the norm, so nearly every
-// tile runs five digits.  Dropping the levels s > D and rounding below the
+// conversion (which writes all six planes).  On the 30-qubit circuit a tile
+// holds about 2^-9 of the norm, so nearly every tile runs five digits.
+// Dropping the levels s > D and rounding below the
 // unit leave errors of about one unit per block.  A pass runs in this form
 // only when all its blocks are unitary.
 constexpr uint32_t kDgPlane = 16384;                       // 128 rows x 64 bf16
@@ -421,6 +421,14 @@ constexpr int kDgLoadIters = 4096 / (2 * kDgThreads);      // amplitude pairs pe
 constexpr int kDgFewDigits = 5;                            // digits of a tile with a small norm
 constexpr uint32_t kDgWarpBound = 1u << 27;                // a warp's norm bound below this: five digits
 static_assert(kDgCols == 8 && kDgLoadIters * 2 == kBlockTableEntries / kDgThreads, "digit kernel thread layout");
+
+// A warp decides from S, the sum of (x 2^-24)^2 over its 256 values x, times 4:
+// the same unit as kDgWarpBound.  x 2^-24 is taken from the value's upper three
+// digits (off by at most 0.51), so the sum of the exact bounds, each at most
+// (257/256)^2 x^2 + 1, is below 1.00785 (S + 32.64 sqrt(S) + 269) + 256, and
+// at least S - 32.64 sqrt(S) - 33: below 2^27 for S under the first limit, at
+// or above it from the second on.  Only between them is the exact bound summed.
+constexpr uint32_t kDgSurelyFive = 132500000u, kDgSurelySix = 134700000u;
 
 // The MMA groups of one block: A plane i against B planes j0 .. j0+nj-1, in
 // issue order; the first group to reach a level initialises it.  Six
@@ -562,32 +570,20 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
 }
 
-// byte j (0..3) of w minus 128, as an exact float: the byte goes into the
-// low mantissa bits of 1.5 * 2^23
-__device__ __forceinline__ float byte_digit(uint32_t w, int j) {
-  return __int_as_float((int)__byte_perm(w, 0x4B400000u, 0x7640u + (uint32_t)j)) - 12583040.0f;
-}
-
-// V = round(x * 2^sh) to nearest, ties to even, |V| < 2^(8D - 1), as D
-// balanced base-256 digits d (d[D-1] the lowest).  A value a digit pass wrote
-// is an integer of the unit already and converts exactly; other values (the
-// first digit pass of a circuit) round once, and ties round to even so that
-// the rounding has no bias (away from zero would grow every tie's
-// magnitude, and the norm with them).  With W = V + 128 (1 + 2^8 + ... +
-// 2^(8(D-1))) every
-// byte of W is its digit plus 128 (the added 128s absorb the borrows), and
-// the top digit is W / 2^(8(D-1)) - 128.  False when |x * 2^sh| >= 2^(8D-1)
-// (the scale does not cover x).
-template <int D>
-__device__ __forceinline__ bool digits_of(double x, int sh, float* d) {
-  static_assert(D == 5 || D == 6, "five or six digits");
+// V = round(x * 2^sh) to nearest, ties to even; false when |x * 2^sh| >= 2^47
+// (the scale does not cover x).  A value a digit pass wrote is an integer of
+// the unit already and converts exactly; other values (the first digit pass of
+// a circuit) round once, and ties round to even so that the rounding has no
+// bias (away from zero would grow every tie's magnitude, and the norm with
+// them).
+__device__ __forceinline__ bool fixed_of(double x, int sh, long long& V) {
   const long long b = __double_as_longlong(x);
   const int ex = (int)((uint32_t)(b >> 52) & 0x7ffu);
   const int k = ex - 1075 + sh;  // |x| 2^sh = m 2^k
-  long long V = 0;
+  V = 0;
   bool ok = true;
   if (ex != 0 && k > -64) {
-    if (k > 8 * D - 54) {
+    if (k > 8 * kDigits - 54) {
       ok = false;
     } else {
       const long long m = (b & 0x000FFFFFFFFFFFFFll) | 0x0010000000000000ll;
@@ -597,18 +593,6 @@ __device__ __forceinline__ bool digits_of(double x, int sh, float* d) {
     }
   }
   if (b < 0) V = -V;
-  const unsigned long long W = (unsigned long long)(V + (D == 6 ? 0x808080808080ll : 0x8080808080ll));
-  const uint32_t wl = (uint32_t)W, wh = (uint32_t)(W >> 32);
-  d[D - 1] = byte_digit(wl, 0);
-  d[D - 2] = byte_digit(wl, 1);
-  d[D - 3] = byte_digit(wl, 2);
-  d[D - 4] = byte_digit(wl, 3);
-  if (D == 6) {
-    d[1] = byte_digit(wh, 0);
-    d[0] = __int_as_float((int)(0x4B400000u | (wh >> 8))) - 12583040.0f;
-  } else {
-    d[0] = __int_as_float((int)(0x4B400000u | wh)) - 12583040.0f;
-  }
   return ok;
 }
 
@@ -643,26 +627,6 @@ __device__ __forceinline__ uint32_t sq_bound_units(double x, int e) {
   if (k >= 0) return min(u2 << k, kDgWarpBound);  // below 2^29 before the min
   if (k <= -19) return 1;
   return (u2 + (1u << -k) - 1) >> -k;
-}
-
-// digits_of for a value already held as its integer V of the unit (the
-// output of the previous digit pass): the same digits, no rounding
-template <int D>
-__device__ __forceinline__ bool digits_of_fixed(long long V, float* d) {
-  const bool ok = V < (1ll << (8 * D - 1)) && V > -(1ll << (8 * D - 1));
-  const unsigned long long W = (unsigned long long)(V + (D == 6 ? 0x808080808080ll : 0x8080808080ll));
-  const uint32_t wl = (uint32_t)W, wh = (uint32_t)(W >> 32);
-  d[D - 1] = byte_digit(wl, 0);
-  d[D - 2] = byte_digit(wl, 1);
-  d[D - 3] = byte_digit(wl, 2);
-  d[D - 4] = byte_digit(wl, 3);
-  if (D == 6) {
-    d[1] = byte_digit(wh, 0);
-    d[0] = __int_as_float((int)(0x4B400000u | (wh >> 8))) - 12583040.0f;
-  } else {
-    d[0] = __int_as_float((int)(0x4B400000u | wh)) - 12583040.0f;
-  }
-  return ok;
 }
 
 // sq_bound_units of x = V 2^(e - 48) from V: the exponent difference ex - e
@@ -709,12 +673,21 @@ struct DgPipe {
   bool range_ok;
 };
 
+// shared-memory offset of digit plane i of a tile in D digits: five digits
+// use the lower five of the six planes
+template <int D>
+__device__ __forceinline__ constexpr uint32_t dg_plane(int i) {
+  return (uint32_t)(i + kDigits - D) * kDgPlane;
+}
+
 // What every tile of the launch shares.
 struct DgFixed {
   unsigned char* sm;
   const Blk5* blk;
   const uint64_t* hoff;
   uint32_t sA, sB, tmem, tlane, bar_b, bar_mma, idesc_base;
+  uint2 load_dest;  // where the loaded amplitudes' digits go
+  int e;            // the state's scale 2^e
   uint64_t free_pos, grid_base;  // next tile's base: ((base | ~free_pos) + grid_base) & free_pos
 };
 
@@ -722,11 +695,12 @@ struct DgFixed {
 // planes j0.. (N = 64 nj) into levels i + j0 .. i + j0 + nj - 1, consecutive
 // 64-column ranges of tensor memory; an initialising group overwrites at
 // K step 0, the others accumulate
+template <int D>
 __device__ __forceinline__ void dg_mma_group(const DgFixed& f, uint32_t sBk, const DgGroup gr) {
   const uint32_t idn = f.idesc_base | ((uint32_t)(8 * gr.nj) << 17);
 #pragma unroll
   for (int ks = 0; ks < 4; ++ks) {
-    const uint64_t ad = sdesc(f.sA + (uint32_t)gr.i * kDgPlane + (uint32_t)ks * 32u);
+    const uint64_t ad = sdesc(f.sA + dg_plane<D>(gr.i) + (uint32_t)ks * 32u);
     const uint64_t bd = sdesc(sBk + (uint32_t)gr.j0 * 8192u + (uint32_t)ks * 32u);
     mma_bf16(f.tmem + 64u * (uint32_t)(gr.i + gr.j0), ad, bd, idn, (gr.init && ks == 0) ? 0u : 1u);
   }
@@ -767,13 +741,110 @@ __device__ __forceinline__ void dg_commit(const DgFixed& f, const DgPassArgs& a,
   }
 }
 
+// a tile's 128 rows of 32 amplitudes (512 contiguous bytes each: the tile
+// holds qubits 0..4) into L2, one 128-byte line per thread of the first 512
+// (per-thread prefetches measured faster than one bulk prefetch per row)
+__device__ __forceinline__ void dg_prefetch(const DgFixed& f, const DgPassArgs& a, uint64_t obase) {
+  const int tid = threadIdx.x;
+  if (tid < 512) {
+    const double2* line = a.s + (obase | ((uint32_t)(tid & 3) * 8u) | f.hoff[tid >> 2]);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(line) : "memory");
+  }
+}
+
+// two adjacent amplitudes (32 aligned bytes) as their bits
+__device__ __forceinline__ void dg_load2(const double2* p, long long* v) {
+  asm volatile("ld.global.cs.v4.b64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
+               : "l"(p));
+}
+
+// The warp's exact verdict: true when the sum of its values' bounds reaches
+// the limit (a thread's own sum is clamped just below it, and flagged when it
+// reaches it, so that the warp sum cannot overflow).
+__device__ __forceinline__ bool dg_exact_verdict(const DgFixed& f, const DgPassArgs& a, uint64_t obase) {
+  uint32_t tb = 0;
+#pragma unroll 1
+  for (int i = 0; i < 4 * kDgLoadIters; ++i) {
+    const uint32_t i0 = (uint32_t)((i >> 2) * kDgThreads + (int)threadIdx.x) * 2u;
+    const double x = __ldcs(reinterpret_cast<const double*>(a.s + (obase | (i0 & 31u) | f.hoff[i0 >> 5])) + (i & 3));
+    tb += a.in_fixed ? sq_bound_units_fixed(__double_as_longlong(x)) : sq_bound_units(x, f.e);
+  }
+  const bool big = tb >= kDgWarpBound;
+  const uint32_t ws = __reduce_add_sync(0xffffffffu, big ? kDgWarpBound - 1 : tb);
+  return __any_sync(0xffffffffu, big) || ws >= kDgWarpBound;
+}
+
+// Loads a tile and writes its digits as the six A planes.  True when the warp
+// asks for six digits: a top digit, or a norm bound at the limit.
+//
+// With W = V + 128 (1 + 2^8 + ... + 2^40) every byte of W is its digit plus
+// 128 (the added 128s absorb the borrows), the top digit W / 2^40 - 128; a byte
+// goes into the low mantissa bits of 1.5 * 2^23, and the real and imaginary
+// digits lose that bias in one packed subtraction.  Five digits are the lower
+// five of the six, so the planes serve both forms.
+//
+// The conversion is bound by issue slots, about 50 instructions per amplitude
+// (106 before, when the norm bound was exact for every value, the parts were
+// unpacked and a six-digit tile converted twice), and by the loads, which
+// take whole 32-byte sectors.  23 passes of a 28-qubit layered circuit (five
+// digits) 130.1 -> 114.2 ms, 8 passes at 26 qubits (six digits) 12.57 -> 10.94.
+__device__ __forceinline__ bool dg_convert(const DgFixed& f, const DgPassArgs& a, DgPipe& p, uint64_t obase,
+                                           bool has_next) {
+  long long v[4 * kDgLoadIters];
+#pragma unroll
+  for (int it = 0; it < kDgLoadIters; ++it) {
+    const uint32_t i0 = (uint32_t)(it * kDgThreads + (int)threadIdx.x) * 2u;
+    dg_load2(a.s + (obase | (i0 & 31u) | f.hoff[i0 >> 5]), v + 4 * it);
+  }
+  if (has_next) dg_prefetch(f, a, ((obase | ~f.free_pos) + f.grid_base) & f.free_pos);
+  if (!a.in_fixed) {
+#pragma unroll
+    for (int i = 0; i < 4 * kDgLoadIters; ++i) p.range_ok &= fixed_of(__longlong_as_double(v[i]), 48 - f.e, v[i]);
+  }
+  uint32_t tops = 0, widest = 0;
+  unsigned long long sq = 0;  // (sum of re^2, sum of im^2) in units of 2^24
+#pragma unroll
+  for (int el = 0; el < 2 * kDgLoadIters; ++el) {
+    const unsigned long long wr = (unsigned long long)(v[2 * el] + 0x808080808080ll);
+    const unsigned long long wi = (unsigned long long)(v[2 * el + 1] + 0x808080808080ll);
+    const uint32_t hr = (uint32_t)(wr >> 40), hi = (uint32_t)(wi >> 40);
+    tops |= (hr ^ 128u) | (hi ^ 128u);
+    widest = max(widest, max(hr, hi));
+    const uint32_t off = dest_at4(f.load_dest, el) << 2;
+    unsigned long long d[kDigits];
+#pragma unroll
+    for (int q = 0; q < kDigits; ++q) {
+      const int j = kDigits - 1 - q;  // byte of W
+      const uint32_t sel = 0x7640u + (uint32_t)(j & 3);
+      const uint32_t br = q == 0 ? 0x4B400000u | hr : __byte_perm((uint32_t)(wr >> (j & 4) * 8), 0x4B400000u, sel);
+      const uint32_t bi = q == 0 ? 0x4B400000u | hi : __byte_perm((uint32_t)(wi >> (j & 4) * 8), 0x4B400000u, sel);
+      unsigned long long b;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "r"(br), "r"(bi));
+      asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d[q]) : "l"(b), "l"(0x4B4000804B400080ull));  // 12583040, twice
+      const uint32_t w = __byte_perm((uint32_t)d[q], (uint32_t)(d[q] >> 32), 0x7632);
+      *reinterpret_cast<uint32_t*>(f.sm + (uint32_t)q * kDgPlane + off) = w;
+    }
+    unsigned long long x;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(d[0]), "l"(0x4380000043800000ull), "l"(d[1]));  // x 256
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(x), "l"(0x4380000043800000ull), "l"(d[2]));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(sq) : "l"(x), "l"(x), "l"(sq));
+  }
+  p.range_ok &= widest <= 256u;
+  const float s4 = 4.0f * (__uint_as_float((uint32_t)sq) + __uint_as_float((uint32_t)(sq >> 32)));
+  const uint32_t ws = __reduce_add_sync(0xffffffffu, __float2uint_ru(fminf(s4, 134217720.0f)));
+  bool six = ws >= kDgSurelySix;
+  if (!six && ws >= kDgSurelyFive) six = dg_exact_verdict(f, a, obase);
+  return six || tops != 0 || !a.five_digits;
+}
+
 // The pass's blocks on one tile whose A planes hold its D digits, then its
 // results (FP64 of unit 2^(e - 48), or the integers themselves for the next
 // digit pass) back to the state.  False when a bounded wait expired (the
 // CTA then stops).
 template <int D>
 __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, DgPipe& p, uint64_t obase,
-                                        bool has_next, int e) {
+                                        bool has_next) {
   const int tid = threadIdx.x;
   unsigned char* sm = f.sm;
   // the tile's first block: every group, after the conversion's barrier
@@ -783,7 +854,7 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
       const uint32_t sBk = f.sB + (p.kimg & 1u) * kDigitImageBytes;
 #pragma unroll
       for (int gi = 0; gi < kDgGroupCount<D>; ++gi) {
-        dg_mma_group(f, sBk, dg_group<D>(gi));
+        dg_mma_group<D>(f, sBk, dg_group<D>(gi));
         if (gi + 1 == kDgFirstStage<D>) mma_commit(f.bar_mma + 8u);
       }
       dg_commit(f, a, p, p.kimg, 0, obase, has_next);
@@ -821,7 +892,7 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
         if (s + 1 <= D - 1) {
 #pragma unroll
           for (int c = 0; c < kDgCplx; ++c)
-            *reinterpret_cast<uint32_t*>(sm + (uint32_t)(s + 1) * kDgPlane + (dest_at4(dest, c) << 2)) =
+            *reinterpret_cast<uint32_t*>(sm + dg_plane<D>(s + 1) + (dest_at4(dest, c) << 2)) =
                 pack_bf16(d[2 * c], d[2 * c + 1]);
         }
       };
@@ -840,7 +911,8 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
       }
 #pragma unroll
       for (int c = 0; c < kDgCplx; ++c)
-        *reinterpret_cast<uint32_t*>(sm + (dest_at4(dest, c) << 2)) = pack_bf16(carry[2 * c], carry[2 * c + 1]);
+        *reinterpret_cast<uint32_t*>(sm + dg_plane<D>(0) + (dest_at4(dest, c) << 2)) =
+            pack_bf16(carry[2 * c], carry[2 * c + 1]);
       fence_proxy_async();
     } else {
       // after the last block the result is V = hi 2^24 + lo, the three
@@ -892,7 +964,7 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
         const uint32_t ie = dest_at4(dest, c);  // the result's tile element
         __stcs(a.s + (obase | (ie & 31u) | f.hoff[ie >> 5]),
                a.out_fixed ? make_double2(__longlong_as_double(vr), __longlong_as_double(vi))
-                           : make_double2(double_of(vr, e - 48), double_of(vi, e - 48)));
+                           : make_double2(double_of(vr, f.e - 48), double_of(vi, f.e - 48)));
       }
     }
     if (tid == 0 && lost && p.issued) p.mma_lost_phase = (int)(k & 1u);
@@ -909,7 +981,7 @@ __device__ __forceinline__ bool dg_tile(const DgPassArgs& a, const DgFixed& f, D
       if (dg_wait_image(f, a, p, k + 1)) {
 #pragma unroll
         for (int gi = 0; gi < kDgGroupCount<D>; ++gi) {
-          dg_mma_group(f, sBn, dg_group<D>(gi));
+          dg_mma_group<D>(f, sBn, dg_group<D>(gi));
           if (gi + 1 == kDgFirstStage<D>) mma_commit(f.bar_mma + 8u);
         }
         dg_commit(f, a, p, k + 1, bi + 1, obase, has_next);
@@ -931,7 +1003,7 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_tblock_dg(const DgPassArgs a)
   // bars[0], bars[1]: image buffers; bars[2]: the MMAs of a block; bars[3]:
   // those of its first stage
   const uint32_t bar_b = smem_u32(&bars[0]), bar_mma = smem_u32(&bars[2]);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -971,8 +1043,8 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_tblock_dg(const DgPassArgs a)
   f.bar_mma = bar_mma;
   // kind::f16: D FP32, A and B BF16, both K-major, M = 128 (N set per MMA)
   f.idesc_base = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
-  const int e = *a.scale_exp + a.scale_shift;
-  const int sh = 48 - e;  // x / 2^e * 2^48 = x * 2^sh: the value in units
+  f.e = *a.scale_exp + a.scale_shift;
+  f.load_dest = my_dests4(a.offsets, blk[0].load_offs);
 
   DgPipe p;
   p.kimg = 0;
@@ -1007,82 +1079,19 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_tblock_dg(const DgPassArgs a)
                      kDigitImageBytes);
     p.b_in_flight |= 1;
   }
-  const uint2 load_dest = my_dests4(a.offsets, blk[0].load_offs);
 
   bool failed = false;
   for (; tile < a.ntiles && !failed; tile += gridDim.x, obase = step_base(obase)) {
     const bool has_next = tile + gridDim.x < a.ntiles;
-    // load: 4 amplitudes per thread, all loads issued first
-    double2 v[2 * kDgLoadIters];
-#pragma unroll
-    for (int it = 0; it < kDgLoadIters; ++it) {
-      const uint32_t i0 = (uint32_t)(it * kDgThreads + tid) * 2u;
-      const double2* src = a.s + (obase | (i0 & 31u) | hoff[i0 >> 5]);
-      v[2 * it] = __ldcs(src);
-      v[2 * it + 1] = __ldcs(src + 1);
-    }
-    // the next tile's 128 rows of 32 amplitudes (512 contiguous bytes each:
-    // the tile holds qubits 0..4) into L2 while this tile computes, one
-    // 128-byte line per thread of the first 512 (per-thread prefetches
-    // measured faster than one bulk prefetch per row: 24.6 against 25.5 ms
-    // per 30-qubit pass)
-    if (tid < 512 && has_next) {
-      const double2* line = a.s + (step_base(obase) | ((uint32_t)(tid & 3) * 8u) | hoff[tid >> 2]);
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(line) : "memory");
-    }
-    // Five digits unless a value needs six or the tile's norm may reach
-    // 2^-9 s: each warp sums its exact bound (a thread's own sum is clamped
-    // just below the bound, and flagged when it reaches it, so that the warp
-    // sum cannot overflow), and the barrier after the conversion ORs the
-    // verdicts.
-    bool six = false;
-    uint32_t tb = 0;
-#pragma unroll
-    for (int el = 0; el < 2 * kDgLoadIters; ++el) {
-      float dr[kDgFewDigits], di[kDgFewDigits];
-      if (a.in_fixed) {
-        const long long vr = __double_as_longlong(v[el].x), vi = __double_as_longlong(v[el].y);
-        six |= !digits_of_fixed<kDgFewDigits>(vr, dr);
-        six |= !digits_of_fixed<kDgFewDigits>(vi, di);
-        tb += sq_bound_units_fixed(vr) + sq_bound_units_fixed(vi);
-      } else {
-        six |= !digits_of<kDgFewDigits>(v[el].x, sh, dr);
-        six |= !digits_of<kDgFewDigits>(v[el].y, sh, di);
-        tb += sq_bound_units(v[el].x, e) + sq_bound_units(v[el].y, e);
-      }
-      const uint32_t off = dest_at4(load_dest, el) << 2;
-#pragma unroll
-      for (int q = 0; q < kDgFewDigits; ++q)
-        *reinterpret_cast<uint32_t*>(sm + (uint32_t)q * kDgPlane + off) = pack_bf16(dr[q], di[q]);
-    }
-    const bool big = tb >= kDgWarpBound;
-    const uint32_t ws = __reduce_add_sync(0xffffffffu, big ? kDgWarpBound - 1 : tb);
-    six |= big || ws >= kDgWarpBound || !a.five_digits;
+    const bool six = dg_convert(f, a, p, obase, has_next);
     fence_proxy_async();
     bool ok;
     if (__syncthreads_or(six ? 1 : 0)) {
-#pragma unroll
-      for (int el = 0; el < 2 * kDgLoadIters; ++el) {
-        float dr[kDigits], di[kDigits];
-        if (a.in_fixed) {
-          p.range_ok &= digits_of_fixed<kDigits>(__double_as_longlong(v[el].x), dr);
-          p.range_ok &= digits_of_fixed<kDigits>(__double_as_longlong(v[el].y), di);
-        } else {
-          p.range_ok &= digits_of<kDigits>(v[el].x, sh, dr);
-          p.range_ok &= digits_of<kDigits>(v[el].y, sh, di);
-        }
-        const uint32_t off = dest_at4(load_dest, el) << 2;
-#pragma unroll
-        for (int q = 0; q < kDigits; ++q)
-          *reinterpret_cast<uint32_t*>(sm + (uint32_t)q * kDgPlane + off) = pack_bf16(dr[q], di[q]);
-      }
-      fence_proxy_async();
-      __syncthreads();
       if (tid == 0) ++tiles_by_digits[1];
-      ok = dg_tile<kDigits>(a, f, p, obase, has_next, e);
+      ok = dg_tile<kDigits>(a, f, p, obase, has_next);
     } else {
       if (tid == 0) ++tiles_by_digits[0];
-      ok = dg_tile<kDgFewDigits>(a, f, p, obase, has_next, e);
+      ok = dg_tile<kDgFewDigits>(a, f, p, obase, has_next);
     }
     if (!ok) failed = true;
   }
@@ -1144,6 +1153,7 @@ void launch_block_pass_digits(State& st, const Blk5* d_blocks, int nblocks, cons
   if (p.K != kBlockTileQubits || st.n < kBlockTileQubits) fail(BF_EINVAL, "internal: block pass needs a 12-qubit tile");
   if (nblocks < 1 || nblocks > kMaxPassBlocks) fail(BF_EINVAL, "internal: block pass of %d blocks", nblocks);
   if (((uintptr_t)d_blocks & 15u) != 0) fail(BF_EINVAL, "internal: block descriptors must be 16-byte aligned");
+  if (((uintptr_t)st.amp & 31u) != 0) fail(BF_EINVAL, "internal: amplitudes must be 32-byte aligned");
   if (((uintptr_t)d_images & 15u) != 0 || ((uintptr_t)d_offsets & 15u) != 0)
     fail(BF_EINVAL, "internal: block images and tables must be 16-byte aligned");
   DgPassArgs a;
