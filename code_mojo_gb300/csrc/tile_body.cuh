@@ -71,9 +71,9 @@ __device__ __forceinline__ void tile_gate(int kind, typename P::Smem* amp, int T
 // at most one fan per Hadamard, multiplied into the pair the Hadamard has in
 // registers anyway: one or two complex products per pair whatever the number
 // of phases.  At 24 qubits, complex128, the value encoding (24 P, 276 CP, 48
-// H) took 4.13 ms as 46 digit blocks in 4 passes and takes 2.25 ms in 3 tile
-// passes with fans; at 27 qubits, complex64, 17.3 against 6.8 ms; the 20-qubit
-// QFT's passes, complex128, 0.30 against 0.15 ms.
+// H) took 4.13 ms as 46 digit blocks in 4 passes and takes 1.64 ms in 3 tile
+// passes with fans; at 27 qubits, complex64, 17.3 against 4.3 ms; the 20-qubit
+// QFT's passes, complex128, 0.30 against 0.11 ms.
 //
 // A phase fan as the CTA holds it: tables in shared memory (the constant
 // folded into one of them), or with neither table the constant alone.

@@ -114,7 +114,7 @@ def tour(n: int, dtype: str, reps: int) -> list[dict]:
     g_ops = OA.OpArray(n, g.ops[n:], g.keep)  # without the initial H layer
     ms = timed(lambda: bfy.execute(st, g_ops, per_gate), stream)
     out.append({"stop": f"{iters} Grover iterations", "kernel": "k_grover_loop", "ms": ms,
-                "bytes_in_S": 2.0 * iters, "GB_per_s": 2.0 * iters * S / (ms * 1e-3) / 1e9})
+                "bytes_in_S": 3.0, "GB_per_s": 3.0 * S / (ms * 1e-3) / 1e9})
     st.close()
     other.close()
     # a batch of small circuits: one persistent launch
