@@ -358,6 +358,9 @@ static double cuda_core_units(const std::vector<TileOp>& ops) {
 // in a double-float tile pass about 2.4 ms).  Measured against 5.0: the
 // 30-qubit circuit 1144 against 1152 ms, value encoding at 22, 24 and 25
 // (fused pairs) qubits 1.95 / 5.25 / 10.8 against 2.47 / 7.00 / 13.6 ms.
+// The digit kernel has become faster since (a 30-qubit pass of 2.5 blocks 19.1
+// instead of 22.2 ms), but 2.1 and 1.8 plan no better: 28-qubit layered 118.9
+// and 119.0 against 118.2 ms, 27 qubits 32.9 and 32.9 against 32.8.
 constexpr double kDigitBlockUnits = 2.5;
 
 // A block pass costs about this many blocks besides its blocks (loading,
