@@ -240,6 +240,13 @@ struct PolF64 {
 
   __device__ static __forceinline__ R from_glob(Glob a) { return R{a.x, a.y}; }
   __device__ static __forceinline__ Glob to_glob(R r) { return make_double2(r.re, r.im); }
+  // whether a pass leaves no room for growth by 2^12 (and 2^7 for a tile's
+  // norm); NaN has none to lose
+  __device__ static __forceinline__ bool large(R r) { return fabs(r.re) >= 0x1p900 || fabs(r.im) >= 0x1p900; }
+  __device__ static __forceinline__ R scaled(R r, int halvings) {
+    const double f = __longlong_as_double((long long)(1023 - halvings) << 52);
+    return R{r.re * f, r.im * f};
+  }
   // times 2^-halvings (exact)
   __device__ static __forceinline__ Glob to_glob_halved(R r, int halvings) {
     const double f = __longlong_as_double((long long)(1023 - halvings) << 52);
@@ -314,6 +321,13 @@ struct PolDF {
   }
   __device__ static __forceinline__ Glob to_glob(R r) {
     return make_double2(df_to_double(r.re), df_to_double(r.im));
+  }
+  __device__ static __forceinline__ bool large(R r) {
+    return fabsf(r.re.hi) >= 0x1p100f || fabsf(r.im.hi) >= 0x1p100f;
+  }
+  __device__ static __forceinline__ R scaled(R r, int halvings) {
+    const float f = __int_as_float((127 - halvings) << 23);
+    return R{dfl{r.re.hi * f, r.re.lo * f}, dfl{r.im.hi * f, r.im.lo * f}};
   }
   __device__ static __forceinline__ Glob to_glob_halved(R r, int halvings) {
     return make_double2(df_to_double(r.re, halvings), df_to_double(r.im, halvings));
@@ -395,6 +409,11 @@ struct PolF32 {
 
   __device__ static __forceinline__ R from_glob(Glob a) { return R{a.x, a.y}; }
   __device__ static __forceinline__ Glob to_glob(R r) { return make_float2(r.re, r.im); }
+  __device__ static __forceinline__ bool large(R r) { return fabsf(r.re) >= 0x1p100f || fabsf(r.im) >= 0x1p100f; }
+  __device__ static __forceinline__ R scaled(R r, int halvings) {
+    const float f = __int_as_float((127 - halvings) << 23);
+    return R{r.re * f, r.im * f};
+  }
   __device__ static __forceinline__ Glob to_glob_halved(R r, int halvings) {
     const float f = __int_as_float((127 - halvings) << 23);
     return make_float2(r.re * f, r.im * f);

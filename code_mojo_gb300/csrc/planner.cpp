@@ -259,7 +259,24 @@ static bool fan_takes(const PhaseTerm& t, uint32_t centre_loc, uint64_t centre_o
   return (l >> a) == 0 || (l & ((1u << a) - 1u)) == 0;
 }
 
+// Hadamards without factors: values grow by up to 2^kMaxHalvings inside a pass
+// (run_tile makes room for it where they are large).
 constexpr int kMaxHalvings = 12;
+
+// |m| of rows and columns 1 and orthogonal, to well above rounding
+static bool is_unitary(const double* m, int dim) {
+  for (int r = 0; r < dim; ++r)
+    for (int c = 0; c <= r; ++c) {
+      double re = 0, im = 0;
+      for (int k = 0; k < dim; ++k) {
+        const double *x = m + 2 * (k * dim + r), *y = m + 2 * (k * dim + c);
+        re += x[0] * y[0] + x[1] * y[1];
+        im += x[0] * y[1] - x[1] * y[0];
+      }
+      if (!(std::fabs(re - (r == c ? 1.0 : 0.0)) <= 1e-6 && std::fabs(im) <= 1e-6)) return false;
+    }
+  return true;
+}
 
 // One table: entry x is the product of the factors whose mask is within x.
 static void fan_table(const std::vector<std::pair<uint32_t, const double*>>& terms, int bits, int shift, double* out) {
@@ -424,14 +441,18 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
   }
   // pairs of Hadamards without their factors: u + v and u - v take 44 of a
   // Hadamard's 72 double-float instructions, and the exact 1/2 per pair costs
-  // the store nothing; at most kMaxHalvings, so that values grow by no more
-  // than 2^kMaxHalvings inside the pass
+  // the store nothing; at most kMaxHalvings, and none in a pass with gates
+  // that may make values grow by themselves
   auto is_h = [](const TileOp& op, bool before) {
     return before ? op.kind != GK_UNITARY && op.um == GK_H : op.kind == GK_H;
   };
   int h = 0;
   for (size_t k = first; k < out.size(); ++k) h += is_h(out[k], true) + is_h(out[k], false);
-  *halvings = std::min(h / 2, kMaxHalvings);
+  auto preserves = [&](const TileOp& op) {
+    if (op.kind == GK_UNITARY) return pool && is_unitary(pool->data() + op.uoff, 1 << op.um);
+    return is_unitary(op.m, 2);
+  };
+  *halvings = h >= 2 && std::all_of(tp.ops.begin(), tp.ops.end(), preserves) ? std::min(h / 2, kMaxHalvings) : 0;
   h = 2 * *halvings;
   for (size_t k = first; k < out.size(); ++k) {
     if (is_h(out[k], true) && h > 0 && h--) out[k].um = GK_HU;

@@ -340,7 +340,11 @@ __host__ __device__ inline size_t tile_fan_bytes(int K) {
 // `smem_raw` also holds the staged matrix.
 // kFans: the ops may carry phase fans; pool then holds their tables and
 // constants, and `smem_raw` also holds the staged ones (tile_smem_bytes).
-// The results are stored times 2^-halvings.
+// The results are stored times 2^-halvings; where an amplitude of the tile is
+// so large that the factor-free Hadamards could leave the arithmetic's range,
+// the tile is scaled before its ops instead: a vote at the barrier that follows
+// the loads, 24-qubit value encoding 1683 against 1674 us without.  (A half at
+// every second of these Hadamards, without a vote: 1775.)
 template <class P, bool kL2Loads = false, bool kUnitaries = false, bool kFans = false>
 __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const TileOp* __restrict__ ops, int nops,
                                          const TileGeom& geo, uint64_t tile, unsigned char* smem_raw,
@@ -408,19 +412,31 @@ __device__ __forceinline__ void run_tile(typename P::Glob* __restrict__ s, const
   const int lowmask = (1 << L) - 1;
   // complex64: two amplitudes per access where qubit 0 is a tile qubit
   const bool words = std::is_same<P, PolF32>::value && L > 0;
+  bool large = false;
   if (words) {
     for (int k = tid; k < (TS >> 1); k += kTileThreads) {
       const uint64_t gi = obase | (uint64_t)((2 * k) & lowmask) | hoff[(2 * k) >> L];
       const float4* p = reinterpret_cast<const float4*>(s + gi);
-      reinterpret_cast<float4*>(amp)[k] = kL2Loads ? __ldcg(p) : *p;
+      const float4 w = kL2Loads ? __ldcg(p) : *p;
+      if constexpr (std::is_same<P, PolF32>::value) large |= P::large(R{w.x, w.y}) || P::large(R{w.z, w.w});
+      reinterpret_cast<float4*>(amp)[k] = w;
     }
   } else {
     for (int e = tid; e < TS; e += kTileThreads) {
       uint64_t gi = obase | (uint64_t)(e & lowmask) | hoff[e >> L];
-      amp[e] = P::to_smem(P::from_glob(kL2Loads ? __ldcg(s + gi) : s[gi]));
+      const R r = P::from_glob(kL2Loads ? __ldcg(s + gi) : s[gi]);
+      large |= P::large(r);
+      amp[e] = P::to_smem(r);
     }
   }
-  __syncthreads();
+  // (the warp reduction makes the branch uniform for the compiler: without it
+  // the op loop keeps its descriptors in per-thread registers, 64 instead of 40)
+  if (__reduce_or_sync(0xffffffffu, (unsigned)__syncthreads_or(large && halvings > 0)) != 0) {
+#pragma unroll 1
+    for (int e = tid; e < TS; e += kTileThreads) amp[e] = P::to_smem(P::scaled(P::from_smem(amp[e]), halvings));
+    halvings = 0;
+    __syncthreads();
+  }
 
   for (int i = 0; i < nops; ++i) {
     const TileOp* op = ops + i;

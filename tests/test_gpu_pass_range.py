@@ -1,0 +1,82 @@
+"""Hadamards of a tile pass run in pairs without their factors: the pass must
+give every amplitude its right power of two, and stay inside FP32's exponent
+range wherever the gates one by one do.  Amplitudes are compared directly, with
+no norm restored and none divided out.
+
+Bound: a gate or phase rounds each amplitude of a pair to a few units of the
+arithmetic (2^-24 at complex64, 2^-45 for a double-float product), so a circuit
+of G ops is off by at most 4 G units of the state's norm."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from code_mojo_gb300 import butterfly as bfy
+from code_mojo_gb300 import workloads as W
+from code_mojo_gb300.batch import Batch
+from oracle import pyoracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def hadamards(n, times):
+    qc = bfy.QuantumCircuit(n)
+    for _ in range(times):
+        for q in range(n):
+            qc.h(q)
+    return qc
+
+
+def qft_gates(n):
+    out = bfy.QuantumCircuit(n)
+    out.transformations = [t for t in W.qft_circuit(n).transformations if isinstance(t, bfy.GateTransformation)]
+    return out
+
+
+CIRCUITS = {
+    "h": lambda n: hadamards(n, 1),          # an odd number of factors at odd n
+    "hh": lambda n: hadamards(n, 2),
+    "hhh": lambda n: hadamards(n, 3),
+    "qft": qft_gates,
+    "encode": lambda n: W.encode_value_circuit(n, 2.7),
+}
+
+
+def off(got, exp):
+    return np.linalg.norm(got - exp) / np.linalg.norm(exp)
+
+
+# 2^120: a pass of 12 pairs has no room for its factors' 2^12
+@pytest.mark.parametrize("scale", [0, 120, -60])
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+@pytest.mark.parametrize("name", list(CIRCUITS))
+@pytest.mark.parametrize("n,K", [(1, 0), (5, 5), (7, 0), (12, 12), (13, 9)])
+def test_amplitudes_keep_their_scale(name, n, K, dtype, scale):
+    qc = CIRCUITS[name](n)
+    re, im = W.random_normal_state(n, 31)
+    if dtype == "c64":
+        re, im = (x.astype(np.float32).astype(np.float64) for x in (re, im))
+    ctx = bfy.ExecContext()
+    ctx.gpu_tile_qubits = K
+    ctx.gpu_tensor_blocks = False
+    ctx.gpu_renormalize = False
+    st = bfy.QuantumState.from_soa(np.ldexp(re, scale), np.ldexp(im, scale), dtype)
+    bfy.execute(st, qc, ctx)
+    gr, gi = st.download()
+    st.close()
+    r, i = O.run(qc, re, im)
+    unit = 2.0 ** -24 if dtype == "c64" else 2.0 ** -45
+    assert off(np.ldexp(gr, -scale) + 1j * np.ldexp(gi, -scale), r + 1j * i) <= 4 * len(qc.transformations) * unit
+
+
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+def test_a_batch_keeps_the_factors(dtype):
+    names = [(k, n) for k in CIRCUITS for n in (1, 6, 11, 13)]
+    b = Batch([CIRCUITS[k](n) for k, n in names], dtype, tile_qubits=9)
+    b.run()
+    for c, (k, n) in enumerate(names):
+        qc = CIRCUITS[k](n)
+        r, i = O.run(qc, *O.basis(n))
+        unit = 2.0 ** -24 if dtype == "c64" else 2.0 ** -45
+        assert off(b.download(c), r + 1j * i) <= 4 * len(qc.transformations) * unit
+    b.close()
