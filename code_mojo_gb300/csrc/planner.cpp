@@ -396,7 +396,9 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
     return joined;
   };
   for (const TileOp& op : tp.ops) {
-    if (op.kind == GK_PHASE) {
+    // (a factor that is not a phase stays by itself: products of several could
+    // leave FP32's range where the gates one by one do not)
+    if (op.kind == GK_PHASE && std::fabs(op.m[6] * op.m[6] + op.m[7] * op.m[7] - 1.0) <= 1e-6) {
       PhaseTerm t;
       t.op = &op;
       t.loc = op.cmask_loc | (op.tloc >= 0 ? 1u << op.tloc : 0u);
@@ -404,7 +406,7 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
       pending.push_back(t);
       continue;
     }
-    if (op.kind == GK_DIAG) {  // commutes with every phase
+    if (op.kind == GK_PHASE || op.kind == GK_DIAG) {  // commutes with every phase
       out.push_back(op);
       continue;
     }

@@ -80,3 +80,29 @@ def test_a_batch_keeps_the_factors(dtype):
         unit = 2.0 ** -24 if dtype == "c64" else 2.0 ** -45
         assert off(b.download(c), r + 1j * i) <= 4 * len(qc.transformations) * unit
     b.close()
+
+
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+@pytest.mark.parametrize("inside", [True, False])
+def test_factors_that_are_no_phases(dtype, inside):
+    """diag(1, 2^60) and diag(1, 2^-60) in turn: every amplitude of the state
+    goes up and comes back, though the product of either kind overflows.  The
+    factors are powers of two, so the amplitudes return exactly."""
+    n = 9
+    qc = bfy.QuantumCircuit(n)
+    up, down = ((1, 2, 3), (5, 6, 7)) if inside else ((8, 7, 6), (1, 2, 3))
+    for a, b in zip(up, down):
+        qc.custom(0, np.diag([1.0, 2.0 ** 60]).astype(complex), [a])
+        qc.custom(0, np.diag([1.0, 2.0 ** -60]).astype(complex), [b])
+    x = np.arange(1 << n)
+    paired = np.all([(x >> a & 1) == (x >> b & 1) for a, b in zip(up, down)], axis=0)
+    re, im = (np.where(paired, v.astype(np.float32), 0.0).astype(np.float64) for v in W.random_normal_state(n, 41))
+    ctx = bfy.ExecContext()
+    ctx.gpu_tile_qubits = 8 if inside else 6
+    ctx.gpu_tensor_blocks = False
+    ctx.gpu_renormalize = False
+    st = bfy.QuantumState.from_soa(re, im, dtype)
+    bfy.execute(st, qc, ctx)
+    gr, gi = st.download()
+    st.close()
+    assert np.array_equal(gr, re) and np.array_equal(gi, im)
