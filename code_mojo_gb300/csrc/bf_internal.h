@@ -311,7 +311,7 @@ struct State {
   int* h_flag = nullptr;
   bool flag_used = false;
   // the state runs in a server slot that shares the GPU with other slots:
-  // kernels whose CTAs wait for one another (Grover loops) stay narrow
+  // kernels whose CTAs wait for one another (Grover loops) are launched in parts
   bool shared_gpu = false;
   // block descriptors and matrix images of tensor-core passes (device) and
   // their pinned staging; uploaded with the tile program

@@ -323,7 +323,7 @@ void launch_grover_diffuser(State& st, const int32_t* q, int32_t nq) {
 //   x -> x + d          (marked),    d = (W_r - W_0) / k
 // with c and d linear in U_0 and W_0.  The host forms the four coefficients
 // (grover_coefficients); the kernel sums the state, meets at one grid barrier
-// and adds c or d.
+// (or ends there, and its second half is a launch of its own) and adds c or d.
 //
 // Bound by memory: one read for the sum, one read and one write for the
 // update (3S; the sum's second read comes from L2 up to about 2^22
@@ -341,6 +341,7 @@ struct LoopArgs {
   double du, dw;          // d = du U_0 + dw W_0
   uint32_t spin_limit;    // polls of 64 ns before a barrier wait gives up
   float4* partial;        // gridDim.x
+  double2* saved;         // the split form: the marked amplitudes before the loop
   unsigned int* bar;      // arrival counter, zero at launch
   int* flag;              // set to 1 when a barrier wait expires
 };
@@ -408,7 +409,8 @@ __device__ __forceinline__ float2 loop_pair(double v) {
   return make_float2(hi, (float)(v - (double)hi));
 }
 
-template <class T>
+enum { kLoopWhole, kLoopSum, kLoopUpdate };  // both halves in one launch, or one each
+template <class T, int kPart>
 __global__ void __launch_bounds__(256) k_grover_loop(T* __restrict__ s, LoopArgs a) {
   __shared__ dfl wr[8], wi[8];
   __shared__ double shift[4];  // c (re, im), d (re, im)
@@ -418,13 +420,18 @@ __global__ void __launch_bounds__(256) k_grover_loop(T* __restrict__ s, LoopArgs
   const unsigned int G = gridDim.x;
   // every CTA reads the marked amplitudes before any CTA writes the state
   if ((int)threadIdx.x < a.nmarked) {
-    const T v = s[a.marked[threadIdx.x]];
-    mk[threadIdx.x] = make_double2((double)v.x, (double)v.y);
+    if constexpr (kPart == kLoopUpdate) {
+      mk[threadIdx.x] = __ldcg(a.saved + threadIdx.x);
+    } else {
+      const T v = s[a.marked[threadIdx.x]];
+      mk[threadIdx.x] = make_double2((double)v.x, (double)v.y);
+      if (kPart == kLoopSum && blockIdx.x == 0) a.saved[threadIdx.x] = mk[threadIdx.x];
+    }
   }
   // eight loads in flight per thread before any use
   constexpr int kU = 8;
   dfl sr{0.f, 0.f}, si{0.f, 0.f};
-  for (uint64_t base = begin + threadIdx.x; base < end; base += kU * blockDim.x) {
+  for (uint64_t base = begin + threadIdx.x; base < end && kPart != kLoopUpdate; base += kU * blockDim.x) {
     T v[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
@@ -439,12 +446,15 @@ __global__ void __launch_bounds__(256) k_grover_loop(T* __restrict__ s, LoopArgs
       si = df_add(si, xi);
     }
   }
-  block_sum2(sr, si, wr, wi);
-  if (threadIdx.x == 0) a.partial[blockIdx.x] = make_float4(sr.hi, sr.lo, si.hi, si.lo);
-  if (G > 1) {
-    if (!loop_barrier(a, G)) return;
-  } else {
-    __syncthreads();
+  if constexpr (kPart != kLoopUpdate) {
+    block_sum2(sr, si, wr, wi);
+    if (threadIdx.x == 0) a.partial[blockIdx.x] = make_float4(sr.hi, sr.lo, si.hi, si.lo);
+    if constexpr (kPart == kLoopSum) return;
+    if (G > 1) {
+      if (!loop_barrier(a, G)) return;
+    } else {
+      __syncthreads();
+    }
   }
   sr = si = dfl{0.f, 0.f};
   for (unsigned int c = threadIdx.x; c < G; c += blockDim.x) {
@@ -522,28 +532,38 @@ static void grover_coefficients(LoopArgs& a, int iters) {
 template <class T>
 static void launch_grover_t(State& st, LoopArgs& a) {
   int per_sm = 0;
-  BF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_grover_loop<T>, 256, 0));
+  BF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_grover_loop<T, kLoopWhole>, 256, 0));
   const uint64_t resident = (uint64_t)std::max(1, per_sm) * (uint64_t)st.num_sms;
-  // a server slot shares the GPU: its CTAs wait for one another at the
-  // barrier, so it takes at most kSharedLoopCtas and the other slots keep the rest
-  constexpr uint64_t kSharedLoopCtas = 16;
-  const uint64_t cap = st.shared_gpu ? kSharedLoopCtas : (uint64_t)2 * st.num_sms;
   // chunks of at least 4096 amplitudes
-  uint64_t G = std::max<uint64_t>(1, std::min<uint64_t>(std::min(cap, resident), st.N >> 12));
+  uint64_t G = std::max<uint64_t>(1, std::min<uint64_t>(std::min((uint64_t)2 * st.num_sms, resident), st.N >> 12));
   a.chunk = (st.N + G - 1) / G;
   a.chunk = (a.chunk + 255) & ~255ull;
   G = (st.N + a.chunk - 1) / a.chunk;
-  // partial sums (G float4), the arrival counter after them
-  const size_t bytes = G * sizeof(float4) + 16;
+  // partial sums (G float4), the marked amplitudes, the arrival counter
+  const size_t bytes = G * sizeof(float4) + sizeof a.marked / sizeof a.marked[0] * sizeof(double2) + 16;
   ensure_partials(st, (bytes + 2 * sizeof(double) - 1) / (2 * sizeof(double)), 0);
   a.partial = reinterpret_cast<float4*>(st.d_partial);
-  a.bar = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(st.d_partial) + G * sizeof(float4));
+  a.saved = reinterpret_cast<double2*>(a.partial + G);
+  a.bar = reinterpret_cast<unsigned int*>(a.saved + sizeof a.marked / sizeof a.marked[0]);
   a.flag = state_flag(st);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)G);
   cfg.blockDim = dim3(256);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st.stream;
+  T* s = static_cast<T*>(st.amp);
+  if (st.shared_gpu && G > 1) {
+    // a server slot shares the GPU: CTAs that wait at a barrier would hold SMs
+    // that the other slots' kernels need, so the two halves are launches of
+    // their own, which wait for nothing.  A request of 26 qubits, complex128,
+    // whatever the count: 4.9 ms; with the barrier and 16 CTAs 11.9 ms; with
+    // the ops one by one 5.8 ms at 2 iterations and 15.3 ms at 16.  At 20
+    // qubits 0.27 ms, 0.37 with 16 CTAs.
+    BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_loop<T, kLoopSum>, s, a));
+    BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_loop<T, kLoopUpdate>, s, a));
+    st.launches += 2;
+    return;
+  }
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
@@ -552,7 +572,7 @@ static void launch_grover_t(State& st, LoopArgs& a) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
   }
-  BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_loop<T>, static_cast<T*>(st.amp), a));
+  BF_CUDA(cudaLaunchKernelEx(&cfg, k_grover_loop<T, kLoopWhole>, s, a));
   st.launches++;
 }
 

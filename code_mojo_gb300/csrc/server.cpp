@@ -143,7 +143,7 @@ static void worker_main(Server* sv, int slot) {
   bool ready = true;
   try {
     init_state_runtime(st);
-    // the slot shares the GPU: a Grover loop takes only part of the SMs
+    // the slot shares the GPU: no kernel whose CTAs wait for one another
     st.shared_gpu = true;
     // small requests on a stream of the highest priority, large ones on a
     // stream of the lowest
