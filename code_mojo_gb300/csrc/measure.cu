@@ -25,18 +25,22 @@ namespace bf {
 constexpr int kMeasThreads = 256;
 constexpr int kMaxOutcomeBits = 20;
 constexpr int kMargTileBits = 11;                                 // 2048 amplitudes: 32 KiB at complex128
+constexpr int kMargCtas = 5;                                      // resident per SM (48 registers)
+constexpr uint64_t kMargHostSums = 2048;
 constexpr int kMargPer = (1 << kMargTileBits) / kMeasThreads;     // tile positions per thread
 
-// Outcome probabilities.  The state is read in contiguous tiles of 2^T
-// amplitudes (its low T index bits), whatever qubits are listed: a CTA owns
-// one setting of the listed free qubits above the tile and walks the settings
-// of the summed-out ones there, each thread adding |amp|^2 to the same eight
-// tile positions in registers.  Only then are the tile's own summed-out bits
-// folded, once, in registers, between lanes and in shared memory (all of them
-// in shared memory cost 16 high qubits of 27, one tile per CTA, 1.01 against
-// 0.83 ms), and the tile's outcomes written.  A long
-// walk is cut into chunks so that the grid fills the GPU; k_marginal_chunks
-// adds the chunks' sums.
+// Outcome probabilities.  The state is read in tiles of 2^T amplitudes: its
+// lowest T index bits that no fixed qubit takes.  A CTA owns one setting of the
+// listed free qubits above the tile and walks the settings of the summed-out
+// ones there, each thread adding |amp|^2 to the same eight tile positions in
+// registers.  Only then are the tile's own summed-out bits folded, once, in
+// registers, between lanes and through shared memory, and the tile's outcomes
+// written.  A long walk is cut into chunks so that the grid fills the GPU; the
+// host or k_marginal_chunks adds the chunks' sums.
+//
+// A tile is contiguous when no fixed qubit lies in its range (kMargRun).  It
+// was contiguous whatever is fixed before, and 11 low fixed qubits of 28 left
+// one live amplitude of 2048 per step: 717 us, 32 like this.
 //
 // Bound by HBM: the state is read once in 32 KiB runs (8 independent 16-byte
 // loads per thread in flight).  One CTA per outcome, which this replaces, read
@@ -44,11 +48,13 @@ constexpr int kMargPer = (1 << kMargTileBits) / kMeasThreads;     // tile positi
 // A 20-qubit register of 24 (complex128): 5.33 ms then, 0.70 ms now, most of
 // it the 8 MiB result's copy; 16 of 28 (complex128): 2.97 against 0.87 ms,
 // 0.72 of the copy bandwidth; 16 of 29 (complex64): 5.22 against 0.87 ms.
+enum { kMargRun, kMargSpread, kMargPart };  // a contiguous tile, a whole one, less than one
 struct MargArgs {
   int32_t tile_bits;       // T
-  uint64_t low_mask;       // listed qubits with a fixed value inside the tile,
-  uint64_t low_val;        // and their required bits
-  uint64_t high_val;       // the fixed qubits' required bits above the tile
+  uint64_t tile_mask;      // the tile's index bits
+  uint64_t row[kMargPer];  // index of tile position j * kMeasThreads
+  int8_t lane_pos[8];      // index bits of the tile's lowest 8 (of all there are)
+  uint64_t fixed_val;      // the fixed qubits' required bits
   uint64_t free_high;      // free listed qubits above the tile
   uint64_t sum_high;       // summed-out qubits above the tile
   uint64_t steps;          // 2^popcount(sum_high)
@@ -56,7 +62,8 @@ struct MargArgs {
   uint32_t chunks;         // CTAs per setting of free_high
   uint64_t outcomes;
   int32_t nfree_low;
-  int8_t low_pos[kMaxOutcomeBits];   // free qubits inside the tile, ascending
+  uint32_t keep;           // their bits in a tile position
+  int8_t low_pos[kMaxOutcomeBits];   // tile positions of the free qubits inside it, ascending
   int8_t low_out[kMaxOutcomeBits];   // their bit in the outcome index
   int8_t high_out[kMaxOutcomeBits];  // outcome bits of free_high, ascending
 };
@@ -74,7 +81,7 @@ __device__ __forceinline__ dfl prob_df<float2>(float2 a) {
 }
 
 // the bits of x spread over the set positions of mask, ascending
-__device__ __forceinline__ uint64_t deposit_mask(uint64_t x, uint64_t mask) {
+__host__ __device__ __forceinline__ uint64_t deposit_mask(uint64_t x, uint64_t mask) {
   uint64_t r = 0;
   for (; x && mask; x >>= 1) {
     const uint64_t low = mask & (0 - mask);
@@ -95,45 +102,50 @@ __device__ __forceinline__ void load_now(float2& v, const float2* p) {
 }
 
 template <class T>
-__global__ void __launch_bounds__(kMeasThreads) k_marginal(const T* __restrict__ s, const MargArgs a,
+__global__ void __launch_bounds__(kMeasThreads, kMargCtas) k_marginal(const T* __restrict__ s, const MargArgs a,
                                                            double* __restrict__ out) {
   __shared__ dfl sum[1 << kMargTileBits];
   const uint64_t h = blockIdx.x / a.chunks, chunk = blockIdx.x % a.chunks;
   const uint32_t size = 1u << a.tile_bits;
-  const uint64_t base = a.high_val | deposit_mask(h, a.free_high);
-  dfl acc[kMargPer];
-  bool live[kMargPer];
+  const bool run = a.tile_mask == (1u << kMargTileBits) - 1u;
+  uint64_t lane = threadIdx.x;
+  if (!run) {
+    lane = 0;
 #pragma unroll
-  for (int j = 0; j < kMargPer; ++j) {
-    const uint32_t e = threadIdx.x + j * kMeasThreads;
-    acc[j] = dfl{0.f, 0.f};
-    live[j] = e < size && (e & a.low_mask) == a.low_val;
+    for (int b = 0; b < 8; ++b) lane |= (uint64_t)((threadIdx.x >> b) & 1u) << a.lane_pos[b];
   }
+  const uint64_t base = a.fixed_val | deposit_mask(h, a.free_high) |
+                        lane;
+  dfl acc[kMargPer];
+#pragma unroll
+  for (int j = 0; j < kMargPer; ++j) acc[j] = dfl{0.f, 0.f};
   const uint64_t first = chunk * a.per_chunk, last = min(first + a.per_chunk, a.steps);
   // the summed-out bits step by masked addition: the ones between them carry
   uint64_t r = deposit_mask(first, a.sum_high);
-  auto walk = [&](auto whole) {
+  auto walk = [&](auto form) {
     for (uint64_t k = first; k < last; ++k, r = ((r | ~a.sum_high) + 1) & a.sum_high) {
-      const T* p = s + (base | r) + threadIdx.x;
+      const T* p = s + (base | r);
       T v[kMargPer];
 #pragma unroll
       for (int j = 0; j < kMargPer; ++j) {
-        if constexpr (!decltype(whole)::value) v[j] = T{};
-        if (decltype(whole)::value || live[j]) load_now(v[j], p + j * kMeasThreads);
+        if constexpr (decltype(form)::value == kMargRun) load_now(v[j], p + j * kMeasThreads);
+        if constexpr (decltype(form)::value == kMargSpread) load_now(v[j], p + a.row[j]);
+        if constexpr (decltype(form)::value == kMargPart) {
+          v[j] = T{};
+          if (threadIdx.x + j * kMeasThreads < size) load_now(v[j], p + a.row[j]);
+        }
       }
 #pragma unroll
       for (int j = 0; j < kMargPer; ++j) acc[j] = df_add(acc[j], prob_df<T>(v[j]));
     }
   };
-  // (a whole tile of unlisted or free low qubits: no conditions on the loads)
-  if (size == (1u << kMargTileBits) && a.low_mask == 0) walk(std::true_type{});
-  else walk(std::false_type{});
+  if (run) walk(std::integral_constant<int, kMargRun>{});
+  else if (a.tile_bits == kMargTileBits) walk(std::integral_constant<int, kMargSpread>{});
+  else walk(std::integral_constant<int, kMargPart>{});
   // Fold the tile bits that are not outcome bits: the three highest between
   // the thread's own sums, the five lowest between the lanes, the three in
   // between through shared memory.
-  uint32_t keep = 0;
-  for (int i = 0; i < a.nfree_low; ++i) keep |= 1u << a.low_pos[i];
-  const uint32_t gone = (size - 1u) & ~keep;
+  const uint32_t gone = (size - 1u) & ~a.keep;
 #pragma unroll
   for (int b = 2; b >= 0; --b) {
     if (!((gone >> (8 + b)) & 1u)) continue;
@@ -141,23 +153,18 @@ __global__ void __launch_bounds__(kMeasThreads) k_marginal(const T* __restrict__
     for (int j = 0; j < kMargPer; ++j)
       if (!((j >> b) & 1)) acc[j] = df_add(acc[j], acc[j | (1 << b)]);
   }
+  for (int b = 0; b < 5; ++b) {
+    if (!((gone >> b) & 1u)) continue;
 #pragma unroll
-  for (int j = 0; j < kMargPer; ++j) {
-    if (((uint32_t)j << 8) & gone) continue;
-    for (int b = 0; b < 5; ++b)
-      if ((gone >> b) & 1u)
+    for (int j = 0; j < kMargPer; ++j)
+      if (!(((uint32_t)j << 8) & gone))
         acc[j] = df_add(acc[j], dfl{__shfl_xor_sync(0xffffffffu, acc[j].hi, 1 << b),
                                     __shfl_xor_sync(0xffffffffu, acc[j].lo, 1 << b)});
-    const uint32_t e = threadIdx.x + j * kMeasThreads;
-    if (e < size && !(threadIdx.x & 31u & gone)) sum[e] = acc[j];
   }
-  uint32_t folded = gone & 0x71fu;  // lane and register bits
-  for (int b = 7; b >= 5; --b) {
-    if (!((gone >> b) & 1u)) continue;
-    folded |= 1u << b;
-    __syncthreads();
-    for (uint32_t e = threadIdx.x; e < size; e += kMeasThreads)
-      if (!(e & folded)) sum[e] = df_add(sum[e], sum[e | (1u << b)]);
+#pragma unroll
+  for (int j = 0; j < kMargPer; ++j) {
+    const uint32_t e = threadIdx.x + j * kMeasThreads;
+    if (e < size && !(e & gone & 0x71fu)) sum[e] = acc[j];
   }
   __syncthreads();
   uint64_t oh = 0;
@@ -169,25 +176,40 @@ __global__ void __launch_bounds__(kMeasThreads) k_marginal(const T* __restrict__
       e |= ((k >> i) & 1u) << a.low_pos[i];
       o |= (uint64_t)((k >> i) & 1u) << a.low_out[i];
     }
-    out[chunk * a.outcomes + o] = (double)sum[e].hi + (double)sum[e].lo;
+    dfl v = sum[e];
+    if (gone & 0xe0u) {
+      dfl w[8];
+#pragma unroll
+      for (uint32_t x = 0; x < 8; ++x) w[x] = (x << 5) & ~gone ? dfl{0.f, 0.f} : sum[e | (x << 5)];
+#pragma unroll
+      for (int half = 4; half > 0; half >>= 1)
+        for (int x = 0; x < half; ++x) w[x] = df_add(w[x], w[x + half]);
+      v = w[0];
+    }
+    out[chunk * a.outcomes + o] = (double)v.hi + (double)v.lo;
   }
 }
 
-// out[o] = sum over chunks of in[c * outcomes + o]: 32 outcomes by 8 chunk
-// lanes per CTA, the lanes' sums added in lane order
+// out[o] = sum over chunks of in[c * outcomes + o]: `width` outcomes (a power
+// of two) by 256 / width chunk lanes per CTA, the lanes' sums folded by halves.
+// The width leaves a lane about eight chunks: with 8 lanes whatever the counts,
+// the 1024 chunks of one outcome at 22 qubits were a chain of 128 loads, and
+// the call took 55 us (30 now).
 __global__ void __launch_bounds__(256) k_marginal_chunks(const double* __restrict__ in, uint64_t outcomes,
-                                                         uint32_t chunks, double* __restrict__ out) {
-  __shared__ double part[8][32];
-  const uint32_t x = threadIdx.x & 31, y = threadIdx.x >> 5;
-  const uint64_t o = (uint64_t)blockIdx.x * 32 + x;
+                                                         uint32_t chunks, uint32_t width, double* __restrict__ out) {
+  __shared__ double part[256];
+  const uint32_t x = threadIdx.x & (width - 1), y = threadIdx.x / width, lanes = 256 / width;
+  const uint64_t o = (uint64_t)blockIdx.x * width + x;
   double acc = 0;
   if (o < outcomes)
-    for (uint32_t c = y; c < chunks; c += 8) acc += in[c * outcomes + o];
-  part[y][x] = acc;
+    for (uint32_t c = y; c < chunks; c += lanes) acc += in[c * outcomes + o];
+  part[threadIdx.x] = acc;
   __syncthreads();
-  if (y != 0 || o >= outcomes) return;
-  for (int k = 1; k < 8; ++k) acc += part[k][x];
-  out[o] = acc;
+  for (uint32_t half = 128; half >= width; half >>= 1) {
+    if (threadIdx.x < half) part[threadIdx.x] += part[threadIdx.x + half];
+    __syncthreads();
+  }
+  if (y == 0 && o < outcomes) out[o] = part[x];
 }
 
 // collapse: keep (and scale) the amplitudes whose listed qubits read `want`
@@ -229,11 +251,15 @@ static void check_qubits(const State& st, const int32_t* q, int32_t nq) {
 // The result stays in the state's pinned buffer until its next reduction.
 const double* marginal_probs(State& st, const int32_t* q, const int8_t* values, int32_t nq, uint64_t* count) {
   check_qubits(st, q, nq);
+  if (nq == 0) {  // the norm
+    const double sum = reduce_norm2(st);
+    st.h_partial[0] = sum;
+    *count = 1;
+    return st.h_partial;
+  }
   MargArgs a;
   std::memset(&a, 0, sizeof a);
-  a.tile_bits = std::min(st.n, kMargTileBits);
-  const uint64_t low = (1ull << a.tile_bits) - 1;
-  uint64_t listed = 0;
+  uint64_t listed = 0, fixed = 0;
   int nfree = 0;
   int out_bit[64];
   for (int i = 0; i < nq; ++i) {
@@ -243,36 +269,49 @@ const double* marginal_probs(State& st, const int32_t* q, const int8_t* values, 
     if (v < 0) {
       if (nfree >= kMaxOutcomeBits) fail(BF_EUNSUPPORTED, "more than %d free measured qubits", kMaxOutcomeBits);
       out_bit[q[i]] = nfree++;
-      if (!(bit & low)) a.free_high |= bit;
     } else {
-      out_bit[q[i]] = -1;
-      a.low_mask |= bit & low;
-      if (v) (bit & low ? a.low_val : a.high_val) |= bit;
+      fixed |= bit;
+      if (v) a.fixed_val |= bit;
     }
   }
   int nfh = 0;
   for (int p = 0; p < st.n; ++p) {
-    if (!((listed >> p) & 1) || out_bit[p] < 0) continue;
-    if (p < a.tile_bits) {
-      a.low_pos[a.nfree_low] = (int8_t)p;
-      a.low_out[a.nfree_low++] = (int8_t)out_bit[p];
-    } else {
+    const uint64_t bit = 1ull << p;
+    if (fixed & bit) continue;
+    const bool free_bit = (listed & bit) != 0;
+    if (a.tile_bits < kMargTileBits) {
+      a.tile_mask |= bit;
+      if (a.tile_bits < 8) a.lane_pos[a.tile_bits] = (int8_t)p;
+      if (free_bit) {
+        a.keep |= 1u << a.tile_bits;
+        a.low_pos[a.nfree_low] = (int8_t)a.tile_bits;
+        a.low_out[a.nfree_low++] = (int8_t)out_bit[p];
+      }
+      ++a.tile_bits;
+    } else if (free_bit) {
+      a.free_high |= bit;
       a.high_out[nfh++] = (int8_t)out_bit[p];
+    } else {
+      a.sum_high |= bit;
     }
   }
-  a.sum_high = (st.N - 1) & ~low & ~listed;
+  for (int j = 0; j < kMargPer; ++j) a.row[j] = deposit_mask((uint64_t)j * kMeasThreads, a.tile_mask);
   a.steps = 1ull << __builtin_popcountll(a.sum_high);
   a.outcomes = 1ull << nfree;
-  // about 8 CTAs per SM in all (2048 threads' worth); a chunk is whole
-  // walk steps, and the chunks' sums stay within 32 MiB
-  uint64_t chunks = std::max<uint64_t>(1, ((uint64_t)st.num_sms * 8) >> nfh);
-  chunks = std::min(std::min(chunks, a.steps), std::max<uint64_t>(1, (1ull << 22) >> nfree));
-  a.per_chunk = (a.steps + chunks - 1) / chunks;
+  // One wave of CTAs; a chunk is whole walk steps, at least one per 512
+  // outcomes it writes (so that the sums stay a fraction of what is read), and
+  // the chunks' sums stay within 32 MiB
+  uint64_t chunks = std::max<uint64_t>(1, ((uint64_t)st.num_sms * (nfh ? 8 : kMargCtas)) >> nfh);
+  chunks = std::min(chunks, std::max<uint64_t>(1, (1ull << 22) >> nfree));
+  a.per_chunk = std::max((a.steps + chunks - 1) / chunks, std::min<uint64_t>(a.steps, ((1ull << a.nfree_low) + 511) / 512));
   a.chunks = (uint32_t)((a.steps + a.per_chunk - 1) / a.per_chunk);
-  // sums of the chunks, then (with more than one) the outcomes
+  // Sums of the chunks, then (with more than one) the outcomes; a few sums are
+  // added on the host, for less than a second launch costs.
   const uint64_t sums = (uint64_t)a.chunks * a.outcomes;
-  ensure_partials(st, (size_t)(sums + a.outcomes + 1) / 2, (size_t)(a.outcomes + 1) / 2);
-  double* fin = a.chunks > 1 ? st.d_partial + sums : st.d_partial;
+  const bool on_host = a.chunks > 1 && sums <= kMargHostSums;
+  const uint64_t read = on_host ? sums : a.outcomes;
+  ensure_partials(st, (size_t)(sums + a.outcomes + 1) / 2, (size_t)(read + 1) / 2);
+  double* fin = a.chunks > 1 && !on_host ? st.d_partial + sums : st.d_partial;
   const dim3 grid((unsigned)((uint64_t)a.chunks << nfh));
   if (st.dtype == BF_C128)
     k_marginal<double2><<<grid, kMeasThreads, 0, st.stream>>>(static_cast<const double2*>(st.amp), a, st.d_partial);
@@ -280,14 +319,17 @@ const double* marginal_probs(State& st, const int32_t* q, const int8_t* values, 
     k_marginal<float2><<<grid, kMeasThreads, 0, st.stream>>>(static_cast<const float2*>(st.amp), a, st.d_partial);
   BF_CUDA(cudaGetLastError());
   st.launches++;
-  if (a.chunks > 1) {
-    k_marginal_chunks<<<(unsigned)((a.outcomes + 31) / 32), 256, 0, st.stream>>>(st.d_partial, a.outcomes, a.chunks,
-                                                                                 fin);
+  if (fin != st.d_partial) {
+    uint32_t width = 1;
+    while (width < 32 && width < a.outcomes && width * a.chunks < 2048) width *= 2;
+    k_marginal_chunks<<<(unsigned)((a.outcomes + width - 1) / width), 256, 0, st.stream>>>(
+        st.d_partial, a.outcomes, a.chunks, width, fin);
     BF_CUDA(cudaGetLastError());
     st.launches++;
   }
-  BF_CUDA(cudaMemcpyAsync(st.h_partial, fin, a.outcomes * sizeof(double), cudaMemcpyDeviceToHost, st.stream));
+  BF_CUDA(cudaMemcpyAsync(st.h_partial, fin, read * sizeof(double), cudaMemcpyDeviceToHost, st.stream));
   sync_state(st);
+  for (uint64_t k = a.outcomes; k < read; ++k) st.h_partial[k & (a.outcomes - 1)] += st.h_partial[k];
   *count = a.outcomes;
   return st.h_partial;
 }
