@@ -1041,18 +1041,27 @@ void HostStage::release() {
   cap = 0;
 }
 
+bool HostStage::reserve(uint64_t count) {
+  const uint64_t want = std::min(count, kHostChunk);
+  if (cap >= want) return true;
+  // no kernel of an earlier download is in flight: each was waited for
+  if (p) cudaFreeHost(p);
+  p = nullptr;
+  cap = 0;
+  try {
+    p = static_cast<double*>(host_alloc((size_t)want * 4 * sizeof(double)));
+  } catch (const Error& e) {
+    if (e.code != BF_ENOMEM) throw;
+    return false;
+  }
+  cap = want;
+  return true;
+}
+
 void HostStage::download(uint64_t count, double* re, double* im, cudaStream_t stream, const Convert& convert) {
   if (count == 0) return;
   for (int k = 0; k < 2; ++k)
     if (!done[k]) BF_CUDA(cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming));
-  const uint64_t want = std::min(count, kHostChunk);
-  if (cap < want) {  // no kernel of an earlier download is in flight: each was waited for
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    cap = 0;
-    p = static_cast<double*>(host_alloc((size_t)want * 4 * sizeof(double)));
-    cap = want;
-  }
   const uint64_t chunks = (count + cap - 1) / cap;
   auto half = [&](uint64_t c, int part) { return p + (2 * (c & 1) + (uint64_t)part) * cap; };
   auto start = [&](uint64_t c) {
@@ -1165,7 +1174,7 @@ static void download_soa(State& st, uint64_t offset, uint64_t count, double* re,
     sync_state(st);
     return;
   }
-  if (by_host_stage(count) && host_pageable(re, im)) {
+  if (by_host_stage(count) && host_pageable(re, im) && st.host_stage.reserve(count)) {
     st.host_stage.download(count, re, im, st.stream, [&](double* r, double* i, uint64_t off, uint64_t cnt) {
       launch_deinterleave(st, r, i, offset + off, cnt);
     });

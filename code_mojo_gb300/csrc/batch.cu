@@ -570,7 +570,8 @@ void batch_sync(Batch& b) {
 }
 
 // Through the pinned staging: one conversion kernel and one host copy for a
-// circuit of up to 2^19 amplitudes.  Several threads may download at once.
+// circuit of up to 2^19 amplitudes; without pinned memory for it, through an
+// ordinary copy.  Several threads may download at once.
 void batch_download(Batch& b, int c, double* re, double* im) {
   if (c < 0 || c >= b.ncirc) fail(BF_EINVAL, "circuit index %d out of range", c);
   batch_sync(b);
@@ -580,8 +581,23 @@ void batch_download(Batch& b, int c, double* re, double* im) {
   auto convert = [&](double* r, double* i, uint64_t off, uint64_t cnt) {
     launch_deinterleave(amps + off * eb, b.dtype, r, i, cnt, b.num_sms, b.stream);
   };
-  std::lock_guard<std::mutex> one(b.download_mutex);
-  b.host_stage.download(N, re, im, b.stream, convert);
+  {
+    std::lock_guard<std::mutex> one(b.download_mutex);
+    if (b.host_stage.reserve(N)) {
+      b.host_stage.download(N, re, im, b.stream, convert);
+      return;
+    }
+  }
+  std::vector<unsigned char> h(N * eb);
+  BF_CUDA(cudaMemcpy(h.data(), amps, N * eb, cudaMemcpyDeviceToHost));
+  auto split = [&](auto* p) {
+    for (uint64_t i = 0; i < N; ++i) {
+      re[i] = (double)p[2 * i];
+      im[i] = (double)p[2 * i + 1];
+    }
+  };
+  if (eb == 16) split(reinterpret_cast<const double*>(h.data()));
+  else split(reinterpret_cast<const float*>(h.data()));
 }
 
 void batch_destroy(Batch* b) { free_batch(b); }

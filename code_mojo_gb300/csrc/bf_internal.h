@@ -258,7 +258,10 @@ struct HostStage {
   double* p = nullptr;
   uint64_t cap = 0;                          // amplitudes per buffer
   cudaEvent_t done[2] = {nullptr, nullptr};  // the last kernel on buffer k
-  // blocks until re and im hold `count` amplitudes
+  // buffers for a transfer of `count` amplitudes; false when the system has no
+  // pinned memory left for them (the transfer then takes another way)
+  bool reserve(uint64_t count);
+  // blocks until re and im hold `count` amplitudes (reserved before)
   void download(uint64_t count, double* re, double* im, cudaStream_t stream, const Convert& convert);
   void release();
 };
