@@ -1062,6 +1062,14 @@ void HostStage::download(uint64_t count, double* re, double* im, cudaStream_t st
   if (count == 0) return;
   for (int k = 0; k < 2; ++k)
     if (!done[k]) BF_CUDA(cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming));
+  // a failure on the way leaves no kernel behind that still writes the buffers
+  struct Drain {
+    cudaStream_t stream;
+    bool armed = true;
+    ~Drain() {
+      if (armed) cudaStreamSynchronize(stream);
+    }
+  } drain{stream};
   const uint64_t chunks = (count + cap - 1) / cap;
   auto half = [&](uint64_t c, int part) { return p + (2 * (c & 1) + (uint64_t)part) * cap; };
   auto start = [&](uint64_t c) {
@@ -1080,6 +1088,7 @@ void HostStage::download(uint64_t count, double* re, double* im, cudaStream_t st
       std::memcpy(im + c * cap, half(c, 1), bytes);
     }
   }
+  drain.armed = false;  // (every chunk's event was waited for)
 }
 
 // Host arrays the DMA engine cannot read directly: ordinary pageable memory.

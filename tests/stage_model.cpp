@@ -95,7 +95,39 @@ static int pinned() {
   return bad ? 1 : 0;
 }
 
+// The second chunk's conversion fails while the stream is busy with the first.
+static int drain() {
+  cudaStream_t s;
+  void* d = nullptr;
+  const size_t big = (size_t)1 << 30;
+  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess || cudaMalloc(&d, big) != cudaSuccess) return 20;
+  const uint64_t count = 2 * kHostChunk;
+  std::vector<double> re(count), im(count);
+  HostStage stage;
+  if (!stage.reserve(count)) return 21;
+  int chunk = 0, rc = 0;
+  bool failed = false;
+  try {
+    stage.download(count, re.data(), im.data(), s, [&](double*, double*, uint64_t, uint64_t) {
+      if (chunk++ == 1) throw Error{BF_ECUDA, "no launch"};
+      for (int k = 0; k < 40; ++k) cudaMemsetAsync(d, k, big, s);  // several milliseconds
+    });
+  } catch (const Error&) {
+    failed = true;
+    if (cudaStreamQuery(s) != cudaSuccess) {
+      std::printf("the download returned with its stream busy\n");
+      rc = 1;
+    }
+  }
+  cudaStreamSynchronize(s);
+  stage.release();
+  cudaFree(d);
+  cudaStreamDestroy(s);
+  return failed ? rc : 22;
+}
+
 int main(int argc, char** argv) {
   if (argc == 2 && !std::strcmp(argv[1], "pinned")) return pinned();
+  if (argc == 2 && !std::strcmp(argv[1], "drain")) return drain();
   return 2;
 }

@@ -32,3 +32,7 @@ def run(model, what):
 
 def test_downloads_without_pinned_memory(model):
     run(model, "pinned")
+
+
+def test_a_failed_download_leaves_nothing_in_flight(model):
+    run(model, "drain")
