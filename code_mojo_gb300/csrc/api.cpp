@@ -945,15 +945,20 @@ class CopyPool {
   }
   // dst[0, bytes) = src[0, bytes) for two pairs of arrays, split over the
   // workers and the caller.  One job at a time (callers on other threads wait
-  // their turn); in a process forked after the pool started, whose workers do
-  // not exist, the caller copies alone.
-  void copy2(void* dst0, const void* src0, void* dst1, const void* src1, size_t bytes) {
-    if (getpid() != pid_) {
+  // their turn, or with `alone_if_busy` copy by themselves); in a process forked
+  // after the pool started, whose workers do not exist, the caller copies alone.
+  void copy2(void* dst0, const void* src0, void* dst1, const void* src1, size_t bytes, bool alone_if_busy = false) {
+    std::unique_lock<std::mutex> one_job(job_m_, std::defer_lock);
+    bool alone = getpid() != pid_;
+    if (!alone) {
+      if (alone_if_busy) alone = !one_job.try_lock();
+      else one_job.lock();
+    }
+    if (alone) {
       std::memcpy(dst0, src0, bytes);
       std::memcpy(dst1, src1, bytes);
       return;
     }
-    std::lock_guard<std::mutex> one_job(job_m_);
     const size_t parts = workers_.size() + 1;
     const size_t part = ((bytes / parts) + 255) & ~(size_t)255;
     {
@@ -1082,7 +1087,7 @@ void HostStage::download(uint64_t count, double* re, double* im, cudaStream_t st
     BF_CUDA(cudaEventSynchronize(done[c & 1]));
     const size_t bytes = std::min(cap, count - c * cap) * sizeof(double);
     if (bytes >= kPoolBytes) {
-      CopyPool::get().copy2(re + c * cap, half(c, 0), im + c * cap, half(c, 1), bytes);
+      CopyPool::get().copy2(re + c * cap, half(c, 0), im + c * cap, half(c, 1), bytes, true);
     } else {
       std::memcpy(re + c * cap, half(c, 0), bytes);
       std::memcpy(im + c * cap, half(c, 1), bytes);

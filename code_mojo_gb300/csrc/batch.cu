@@ -14,8 +14,11 @@
 // every state, then all tasks) is captured once into a CUDA graph and
 // replayed by bf_batch_run.
 #include <algorithm>
+#include <condition_variable>
 #include <cstring>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 #include "tile_body.cuh"
@@ -147,6 +150,13 @@ struct BatchTuneRow {
   double ms;  // one run of the sample batch
 };
 
+constexpr size_t kBatchStages = 8;  // of up to 16 MiB each
+// Circuits of up to this many bytes are copied directly.  complex64, whose half
+// the bytes count: 14 qubits 23 us against 31 staged, 16 qubits 55 against 79,
+// 17 qubits 96 against 73.  complex128: 11 qubits 15.6 against 16.8, 13 qubits
+// 22.1 against 22.4, 15 qubits 47 against 46, 17 qubits 156 against 73.
+constexpr size_t kBatchDirect64 = 1u << 19, kBatchDirect128 = 1u << 16;
+
 struct Batch {
   int device = 0, num_sms = 0;
   int dtype = BF_C64, prec = PREC_F32;
@@ -172,8 +182,12 @@ struct Batch {
   cudaStream_t stream = nullptr;
   cudaGraphExec_t graph = nullptr;
   uint64_t launches = 0;
-  HostStage host_stage;
-  std::mutex download_mutex;  // the staging's user
+  // staging for downloads, one per thread that downloads at the same time, up
+  // to kBatchStages (then threads wait); free ones in `idle`
+  std::vector<std::unique_ptr<HostStage>> stages;
+  std::vector<HostStage*> idle;
+  std::mutex stage_mutex;
+  std::condition_variable stage_free;
   // autotuning record: per qubit count, the candidate tile widths timed on a
   // sample of the batch's circuits of that size, and the width chosen
   std::vector<BatchTuneRow> tuning;
@@ -258,7 +272,7 @@ static void free_batch(Batch* b) {
   cudaFree(b->d_ticket);
   cudaFree(b->d_error);
   if (b->h_error) cudaFreeHost(b->h_error);
-  b->host_stage.release();
+  for (auto& s : b->stages) s->release();
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }
@@ -569,9 +583,37 @@ void batch_sync(Batch& b) {
   if (*b.h_error) fail(BF_ETIMEDOUT, "batch: a task waited past its bound for its circuit's previous pass");
 }
 
-// Through the pinned staging: one conversion kernel and one host copy for a
-// circuit of up to 2^19 amplitudes; without pinned memory for it, through an
-// ordinary copy.  Several threads may download at once.
+// A staging of the batch's, for one download.
+class BatchStage {
+ public:
+  explicit BatchStage(Batch& b) : b_(b) {
+    std::unique_lock<std::mutex> lk(b.stage_mutex);
+    if (b.idle.empty() && b.stages.size() < kBatchStages) {
+      b.stages.push_back(std::make_unique<HostStage>());
+      b.idle.push_back(b.stages.back().get());
+    }
+    b.stage_free.wait(lk, [&] { return !b.idle.empty(); });
+    s_ = b.idle.back();
+    b.idle.pop_back();
+  }
+  ~BatchStage() {
+    {
+      std::lock_guard<std::mutex> lk(b_.stage_mutex);
+      b_.idle.push_back(s_);
+    }
+    b_.stage_free.notify_one();
+  }
+  HostStage* operator->() { return s_; }
+
+ private:
+  Batch& b_;
+  HostStage* s_;
+};
+
+// Through a pinned staging: one conversion kernel and one host copy for a
+// circuit of up to 2^19 amplitudes; small circuits, and without pinned memory
+// all, through an ordinary copy.  Threads download side by side (17 qubits,
+// complex128, 8 threads: 44 us each, 82 when they took turns on one staging).
 void batch_download(Batch& b, int c, double* re, double* im) {
   if (c < 0 || c >= b.ncirc) fail(BF_EINVAL, "circuit index %d out of range", c);
   batch_sync(b);
@@ -581,10 +623,10 @@ void batch_download(Batch& b, int c, double* re, double* im) {
   auto convert = [&](double* r, double* i, uint64_t off, uint64_t cnt) {
     launch_deinterleave(amps + off * eb, b.dtype, r, i, cnt, b.num_sms, b.stream);
   };
-  {
-    std::lock_guard<std::mutex> one(b.download_mutex);
-    if (b.host_stage.reserve(N)) {
-      b.host_stage.download(N, re, im, b.stream, convert);
+  if (N * eb > (b.dtype == BF_C128 ? kBatchDirect128 : kBatchDirect64)) {
+    BatchStage stage(b);
+    if (stage->reserve(N)) {
+      stage->download(N, re, im, b.stream, convert);
       return;
     }
   }
