@@ -12,6 +12,7 @@
 #include <thread>
 #include <vector>
 
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include "bf_internal.h"
@@ -1025,15 +1026,34 @@ class CopyPool {
 // copies alone, which costs less than waking the pool.
 //
 // A state's download takes this way below 2^14 amplitudes, where launches and
-// events are the cost (9 qubits 15.8 against 31.5 us, 13 qubits 24 against
-// 31 us), and from 2^18 up to the chunked path, where the arrays are often
-// pages the GPU has not translated yet and the driver's copy into them ranges
-// from 1.0 to 7 ms at 20 qubits (0.51 ms this way, whatever the pages; 0.33
-// against 0.30 ms into arrays the GPU wrote before).  Between them the
-// driver's copy is the faster one (16 qubits 36 against 79 us).
+// events are the cost (9 qubits 15.8 against 31.5 us, 13 qubits 23 against
+// 29 us), and from 2^18 up to the chunked path where the arrays are pages that
+// nothing has touched yet (a new np.empty): the driver's copy takes 0.9 to
+// 2.2 ms into those at 19 to 21 qubits, 0.2 to 0.6 ms this way, but 51 to 214
+// us against 92 to 400 into arrays in use.  Between them the driver's copy is
+// the faster one (16 qubits 36 against 79 us).
 constexpr size_t kPoolBytes = 1u << 20;
-static bool by_host_stage(uint64_t count) {
-  return count < (1ull << 14) || (count >= (1ull << 18) && count < (1ull << 22));
+
+// Whether the arrays' pages are mostly not there yet, by the sixteen in the
+// middle of either array.  (A call costs about 1 us, so two are made; eight
+// places looked at took 6 us, of 51 for a download of 18 qubits.)
+static bool pages_missing(const void* re, const void* im, size_t bytes) {
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE), window = 16;
+  size_t total = 0, missing = 0;
+  for (const void* p : {re, im}) {
+    const uintptr_t lo = (uintptr_t)p / page, pages = ((uintptr_t)p + bytes + page - 1) / page - lo;
+    const size_t n = std::min<size_t>(window, pages);
+    unsigned char there[window];
+    if (mincore((void*)((lo + (pages - n) / 2) * page), n * page, there) != 0) return false;
+    total += n;
+    for (size_t i = 0; i < n; ++i) missing += !(there[i] & 1);
+  }
+  return 2 * missing > total;
+}
+
+static bool by_host_stage(uint64_t count, const void* re, const void* im) {
+  if (count < (1ull << 14)) return true;
+  return count >= (1ull << 18) && count < (1ull << 22) && pages_missing(re, im, count * sizeof(double));
 }
 
 void HostStage::release() {
@@ -1188,7 +1208,7 @@ static void download_soa(State& st, uint64_t offset, uint64_t count, double* re,
     sync_state(st);
     return;
   }
-  if (by_host_stage(count) && host_pageable(re, im) && st.host_stage.reserve(count)) {
+  if (by_host_stage(count, re, im) && host_pageable(re, im) && st.host_stage.reserve(count)) {
     st.host_stage.download(count, re, im, st.stream, [&](double* r, double* i, uint64_t off, uint64_t cnt) {
       launch_deinterleave(st, r, i, offset + off, cnt);
     });

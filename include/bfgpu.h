@@ -199,9 +199,10 @@ int bf_state_set_basis(bf_state* st, uint64_t idx);
  * conversion.  Transfers of at least one chunk from or to pageable arrays
  * go through the state's pinned host buffers (128 MiB, allocated on first
  * use), filled or drained by a pool of library host threads while the DMA
- * engine moves the other chunk.  Downloads of less than 2^14 and of 2^18 to
- * 2^22 amplitudes into pageable arrays are converted straight into pinned
- * buffers that the state keeps, and copied from there by host threads. */
+ * engine moves the other chunk.  Downloads of less than 2^14 amplitudes into
+ * pageable arrays, and of 2^18 to 2^22 into arrays whose pages are mostly
+ * untouched, are converted straight into pinned buffers that the state keeps,
+ * and copied from there by host threads. */
 int bf_state_upload_soa(bf_state* st, const double* re, const double* im);
 int bf_state_download_soa(bf_state* st, double* re, double* im);
 /* Copies amplitudes [offset, offset+count) to host SoA arrays (blocks). */

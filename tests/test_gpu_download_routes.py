@@ -39,3 +39,20 @@ def test_a_batch_read_by_many_threads(dtype):
         t.join()
     b.close()
     assert not bad
+
+
+# 2^18 to 2^22 amplitudes: staged into untouched pages, copied by the driver
+# into touched ones
+@pytest.mark.parametrize("n", [17, 18, 20, 21])
+def test_touched_and_untouched_arrays(n):
+    N = 1 << n
+    re, im = W.random_normal_state(n, n)
+    st = bfy.QuantumState.from_soa(re, im)
+    touched = [lambda: np.empty(N), lambda: np.ones(N), lambda: np.concatenate([np.ones(N // 2), np.empty(N // 2)]),
+               lambda: np.empty(N + 1)[1:]]
+    for a in touched:
+        for b in touched:
+            gr, gi = a(), b()
+            F.check(F.lib().bf_state_download_soa(st.handle, gr.ctypes.data, gi.ctypes.data))
+            assert np.array_equal(gr, re) and np.array_equal(gi, im)
+    st.close()
