@@ -106,3 +106,21 @@ def test_factors_that_are_no_phases(dtype, inside):
     gr, gi = st.download()
     st.close()
     assert np.array_equal(gr, re) and np.array_equal(gi, im)
+
+
+@pytest.mark.parametrize("n", [9, 12, 15, 18, 20])
+def test_complex64_value_encoding_stays_near_fp32(n):
+    """About three roundings of half a unit per Hadamard and its fan along the
+    way of an amplitude, 2 n of them: as a random walk sqrt(6 n) units of 2^-24
+    at three standard deviations, and one for the stored value; in the largest
+    amplitude and in the norm of the error alike."""
+    bound = (np.sqrt(6 * n) + 1) * 2.0 ** -24
+    for v in (0.37, 2 ** (n - 1) + 0.5, 2 ** n - 1.21):
+        qc = W.encode_value_circuit(n, v)
+        st = bfy.QuantumState(n, "c64")
+        bfy.execute(st, qc)
+        got = st.to_complex()
+        st.close()
+        r, i = O.run(qc, *O.basis(n))
+        d = got - (r + 1j * i)
+        assert np.max(np.abs(d)) <= bound and np.linalg.norm(d) <= bound
