@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <deque>
 
 #include "bf_internal.h"
 
@@ -165,11 +166,11 @@ static void gate_matrix(int kind, double a, const double* mat, double* m) {
   }
 }
 
-static void split_pairs(GateInstr& g) {
+static void split_pairs(const double* m, float* mhl) {
   for (int i = 0; i < 8; ++i) {
-    float hi = (float)g.m[i];
-    g.mhl[2 * i] = hi;
-    g.mhl[2 * i + 1] = (float)(g.m[i] - (double)hi);
+    float hi = (float)m[i];
+    mhl[2 * i] = hi;
+    mhl[2 * i + 1] = (float)(m[i] - (double)hi);
   }
 }
 
@@ -200,7 +201,7 @@ GateInstr lower_gate(const bf_op& o, uint32_t spec) {
   } else {
     g.kind = m[1] == 0 ? GK_DENSE_R : GK_DENSE;  // U3: m00 = cos(theta/2) is real
   }
-  split_pairs(g);
+  split_pairs(g.m, g.mhl);
   return g;
 }
 
@@ -241,6 +242,113 @@ struct PhaseTerm {
   const TileOp* op;
   uint32_t loc;
   uint64_t out;
+};
+
+// a diagonal factor that may join a fan: products of several others could leave
+// FP32's range where the gates one by one do not
+static bool unit_factor(const double* m) { return std::fabs(m[6] * m[6] + m[7] * m[7] - 1.0) <= 1e-6; }
+
+// A number per qubit mask (open addressing; 0 for a mask not seen before).
+class MaskTable {
+ public:
+  uint32_t& operator[](uint64_t mask) {  // (mask != 0)
+    if (2 * used_ >= keys_.size()) grow();
+    const size_t i = find(mask);
+    if (keys_[i] == 0) {
+      keys_[i] = mask;
+      ++used_;
+    }
+    return vals_[i];
+  }
+
+ private:
+  size_t find(uint64_t mask) const {
+    size_t i = (size_t)((mask * 0x9e3779b97f4a7c15ull) >> 32) & (keys_.size() - 1);
+    while (keys_[i] != 0 && keys_[i] != mask) i = (i + 1) & (keys_.size() - 1);
+    return i;
+  }
+  void grow() {
+    std::vector<uint64_t> k(keys_.empty() ? 256 : 2 * keys_.size(), 0);
+    std::vector<uint32_t> v(k.size(), 0);
+    k.swap(keys_);
+    v.swap(vals_);
+    for (size_t o = 0; o < k.size(); ++o)
+      if (k[o] != 0) {
+        const size_t i = find(k[o]);
+        keys_[i] = k[o];
+        vals_[i] = v[o];
+      }
+  }
+  std::vector<uint64_t> keys_;
+  std::vector<uint32_t> vals_;
+  size_t used_ = 0;
+};
+
+// The phases of a pass that wait for a gate on one of their qubits: one per
+// mask, so that what waits (and the constants of a fan) is bounded by the
+// masks that differ, and found by tile bit, so that a gate looks at the phases
+// it meets and at no others.  (With a list of all, rescanned at every gate, a
+// pass of 40,000 gates took 590 ms to plan, now 7.5.)
+class PendingPhases {
+ public:
+  explicit PendingPhases(const TilePass& tp) : q_(tp.q) {}
+  void add(const PhaseTerm& t) {
+    uint64_t mask = t.out;
+    for (uint32_t b = t.loc; b; b &= b - 1) mask |= 1ull << q_[__builtin_ctz(b)];
+    uint32_t& id = at_[mask];  // 1 + the latest term of the mask
+    if (id != 0 && live_[id - 1]) {
+      TileOp*& own = own_[id - 1];
+      if (!own) {
+        ops_.push_back(*terms_[id - 1].op);
+        terms_[id - 1].op = own = &ops_.back();
+      }
+      const double r = own->m[6] * t.op->m[6] - own->m[7] * t.op->m[7];
+      own->m[7] = own->m[6] * t.op->m[7] + own->m[7] * t.op->m[6];
+      own->m[6] = r;
+      split_pairs(own->m, own->mhl);
+      return;
+    }
+    id = (uint32_t)terms_.size() + 1;
+    for (uint32_t b = t.loc; b; b &= b - 1) by_bit_[__builtin_ctz(b)].push_back(id - 1);
+    terms_.push_back(t);
+    own_.push_back(nullptr);
+    live_.push_back(1);
+  }
+  // removes the phases on a bit of x (~0: all), in order of arrival
+  std::vector<PhaseTerm> take(uint32_t x) {
+    std::vector<uint32_t> ids;
+    if (x == ~0u) {
+      for (uint32_t i = 0; i < terms_.size(); ++i)
+        if (live_[i]) ids.push_back(i);
+    } else {
+      for (; x; x &= x - 1) {
+        std::vector<uint32_t>& l = by_bit_[__builtin_ctz(x)];
+        for (uint32_t i : l)
+          if (live_[i]) {
+            live_[i] = 0;
+            ids.push_back(i);
+          }
+        l.clear();
+      }
+      std::sort(ids.begin(), ids.end());
+    }
+    std::vector<PhaseTerm> out;
+    out.reserve(ids.size());
+    for (uint32_t i : ids) {
+      out.push_back(terms_[i]);
+      live_[i] = 0;
+    }
+    return out;
+  }
+
+ private:
+  const int32_t* q_;
+  std::deque<TileOp> ops_;  // products of several phases of a mask
+  std::vector<PhaseTerm> terms_;
+  std::vector<TileOp*> own_;  // a term's product in ops_, null while it is one op of the pass
+  std::vector<char> live_;
+  MaskTable at_;
+  std::vector<uint32_t> by_bit_[32];  // terms by tile bit; taken ones drop out when read
 };
 
 // A fan needs at least this many phases: one alone touches a quarter or half
@@ -311,7 +419,7 @@ static void fan_table(const std::vector<std::pair<uint32_t, const double*>>& ter
 int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<double>* pool, int* halvings) {
   const size_t first = out.size();
   const int K = tp.K, a = K / 2;
-  std::vector<PhaseTerm> pending;
+  PendingPhases pending(tp);
   int fans = 0;
   std::vector<uint32_t> fan_bits(1, 0u);  // by fan: the tile bits of its phases
   // fills op's fan from the terms around one centre
@@ -354,18 +462,15 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
       uint32_t cl = centre;
       uint64_t co = 0;
       if (!centre) {
-        int best = 0;
-        for (int q = 0; q < K + 64; ++q) {  // tile bits, then outside qubits
-          const uint32_t l = q < K ? 1u << q : 0u;
-          const uint64_t o = q < K ? 0ull : 1ull << (q - K);
-          int cnt = 0;
-          for (const PhaseTerm& t : terms)
-            cnt += ((t.loc & l) || (t.out & o)) && fan_takes(t, l, o, a);
-          if (cnt > best) {
-            best = cnt;
-            cl = l;
-            co = o;
-          }
+        int cnt[32 + 64] = {};  // tile bits, then outside qubits
+        for (const PhaseTerm& t : terms) {
+          for (uint32_t b = t.loc; b; b &= b - 1) cnt[__builtin_ctz(b)] += fan_takes(t, b & (0u - b), 0, a);
+          for (uint64_t b = t.out; b; b &= b - 1) cnt[32 + __builtin_ctzll(b)] += fan_takes(t, 0, b & (0ull - b), a);
+        }
+        const int best = (int)(std::max_element(cnt, cnt + 96) - cnt);
+        if (cnt[best] > 0) {
+          cl = best < 32 ? 1u << best : 0u;
+          co = best < 32 ? 0ull : 1ull << (best - 32);
         }
       }
       std::vector<PhaseTerm> in, rest;
@@ -396,14 +501,12 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
     return joined;
   };
   for (const TileOp& op : tp.ops) {
-    // (a factor that is not a phase stays by itself: products of several could
-    // leave FP32's range where the gates one by one do not)
-    if (op.kind == GK_PHASE && std::fabs(op.m[6] * op.m[6] + op.m[7] * op.m[7] - 1.0) <= 1e-6) {
+    if (op.kind == GK_PHASE && unit_factor(op.m)) {
       PhaseTerm t;
       t.op = &op;
       t.loc = op.cmask_loc | (op.tloc >= 0 ? 1u << op.tloc : 0u);
       t.out = op.cmask_out | (op.tloc < 0 ? 1ull << op.tglob : 0ull);
-      pending.push_back(t);
+      pending.add(t);
       continue;
     }
     if (op.kind == GK_PHASE || op.kind == GK_DIAG) {  // commutes with every phase
@@ -412,15 +515,13 @@ int merge_phases(const TilePass& tp, std::vector<TileOp>& out, std::vector<doubl
     }
     const bool uni = op.kind == GK_UNITARY;
     const uint32_t x = uni ? ((1u << op.um) - 1u) << op.tloc : 1u << op.tloc;
-    std::vector<PhaseTerm> met, rest;
-    for (const PhaseTerm& t : pending) (t.loc & x ? met : rest).push_back(t);
-    pending.swap(rest);
+    const std::vector<PhaseTerm> met = pending.take(x);
     TileOp g = op;
     const bool joins = !uni && op.kind != GK_SWAP && !op.cmask_loc && !op.cmask_out;
     if (!met.empty()) flush(met, uni ? 0u : x, joins ? &g : nullptr);
     out.push_back(g);
   }
-  flush(pending, 0u, nullptr);
+  flush(pending.take(~0u), 0u, nullptr);
   // A Hadamard goes into the next op on its target where that has a fan and
   // nothing between them touches the target: the pair is read and written once.
   auto touches = [&](const TileOp& op) {
@@ -535,7 +636,9 @@ static int pass_blocks(const std::vector<const GateInstr*>& remaining, uint64_t 
 static double pass_core_units(const std::vector<const GateInstr*>& remaining, uint64_t inQ, uint64_t all) {
   uint64_t blockedX = 0, blockedAll = 0;
   double u = 0;
-  std::vector<uint64_t> pending;
+  // the phases that wait for a gate, one per mask (1: waiting), by qubit
+  std::vector<uint64_t> by_qubit[64];
+  MaskTable pending;
   for (const GateInstr* g : remaining) {
     const uint64_t Xg = gate_xmask(*g);
     const uint64_t Ag = gate_amask(*g);
@@ -545,18 +648,25 @@ static double pass_core_units(const std::vector<const GateInstr*>& remaining, ui
       if ((blockedX & all) == all) break;
       continue;
     }
-    if (g->kind == GK_PHASE) {
-      pending.push_back(Ag);
+    if (g->kind == GK_PHASE && unit_factor(g->m)) {
+      uint32_t& waits = pending[Ag];
+      if (!waits)
+        for (uint64_t b = Ag; b; b &= b - 1) by_qubit[__builtin_ctzll(b)].push_back(Ag);
+      waits = 1;
       continue;
     }
     u += core_units(g->kind, g->um);
     if (!Xg) continue;
-    size_t kept = 0, met = 0;
-    for (uint64_t p : pending) {
-      if (p & Xg) ++met;
-      else pending[kept++] = p;
+    size_t met = 0;
+    for (uint64_t b = Xg; b; b &= b - 1) {
+      std::vector<uint64_t>& l = by_qubit[__builtin_ctzll(b)];
+      for (uint64_t p : l) {
+        uint32_t& waits = pending[p];
+        met += waits;
+        waits = 0;
+      }
+      l.clear();
     }
-    pending.resize(kept);
     if (met >= (size_t)kMinFanTerms) u += core_units(GK_FAN, 0);
     else if (met) u += core_units(GK_PHASE, 0);
   }
@@ -601,8 +711,11 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
     int nQ = L;
     // the qubits the remaining gates touch: once the deferred gates act
     // non-diagonally on all of them, no later gate can join a pass
-    uint64_t all = 0;
-    for (const GateInstr* g : remaining) all |= gate_amask(*g);
+    uint64_t all = 0, all_x = 0;  // all_x: the qubits they act on non-diagonally
+    for (const GateInstr* g : remaining) {
+      all |= gate_amask(*g);
+      all_x |= gate_xmask(*g);
+    }
     {
       uint64_t blockedX = 0, blockedAll = 0;
       for (const GateInstr* g : remaining) {
@@ -628,8 +741,7 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
     }
     bool blocks_chosen = false;
     if (nQ == K && K < n) {
-      uint64_t targets = 0;
-      for (const GateInstr* g : remaining) targets |= gate_xmask(*g);
+      const uint64_t targets = all_x;
       auto search = [&](uint64_t start, auto score) {
         uint64_t set = start;
         double best = score(set);
@@ -673,32 +785,29 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
       }
       if (!blocks_chosen) inQ = by_work;
     }
+    // deferred: those passed over up to `tail`, from where no gate can join
     std::vector<const GateInstr*> taken, deferred;
     std::vector<size_t> taken_at, deferred_at;  // their places in `remaining`
+    size_t tail = 0;
     {
       uint64_t blockedX = 0, blockedAll = 0;
-      size_t i = 0;
-      for (; i < remaining.size(); ++i) {
-        const GateInstr* g = remaining[i];
+      for (; tail < remaining.size(); ++tail) {
+        const GateInstr* g = remaining[tail];
         const uint64_t Xg = gate_xmask(*g);
         const uint64_t Ag = gate_amask(*g);
         if (!(Xg & blockedAll) && !(Ag & blockedX) && !(Xg & ~inQ)) {
           taken.push_back(g);
-          taken_at.push_back(i);
+          taken_at.push_back(tail);
         } else {
           deferred.push_back(g);
-          deferred_at.push_back(i);
+          deferred_at.push_back(tail);
           blockedX |= Xg;
           blockedAll |= Ag;
           if ((blockedX & all) == all) {
-            ++i;
+            ++tail;
             break;
           }
         }
-      }
-      for (; i < remaining.size(); ++i) {
-        deferred.push_back(remaining[i]);
-        deferred_at.push_back(i);
       }
     }
     // A phase that no gate of this pass meets goes back when a deferred gate
@@ -708,6 +817,7 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
     if (!blocks_chosen) {
       uint64_t later = 0, met = 0;
       for (const GateInstr* g : deferred) later |= gate_xmask(*g);
+      for (size_t i = tail; i < remaining.size() && later != all_x; ++i) later |= gate_xmask(*remaining[i]);
       std::vector<char> back(taken.size(), 0);
       bool any = false;
       for (size_t k = taken.size(); k-- > 0;) {
@@ -779,6 +889,7 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
       for (const GateInstr* g : taken) st.tile.ops.push_back(to_tile_op(*g, loc_of));
       steps.push_back(std::move(st));
     }
+    deferred.insert(deferred.end(), remaining.begin() + (std::ptrdiff_t)tail, remaining.end());
     remaining.swap(deferred);
   }
   return steps;
