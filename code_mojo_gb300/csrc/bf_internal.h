@@ -153,21 +153,21 @@ struct TileOp {
                       // Hadamard of the same target that goes before the fan
                       // (GK_H or GK_HU, 0: none)
   int32_t uoff;       // GK_UNITARY: offset (in doubles) of its matrix in the
-                      // program's pool
+                      // program's pool (an op with a fan: the planner's)
   // The phase fan applied before the op (alone for GK_FAN): the product of
   // the phases that share the centre qubit tloc, on the amplitudes whose
   // centre bit is 1 (tloc < 0: the centre is in cmask_out, every amplitude).
   // The phase of local index x is A[x mod 2^a] * B[x >> a] * c, with tables
   // over the tile's low a and other K - a bits and c the product of the
   // entries (mask, factor) whose outside qubits are all 1 in the CTA.
-  int32_t fan;        // 0: none; else 1 + its constant's slot in the pass
+  int32_t fan;        // 0: none; else 1 + its constant's slot in the pass (1 without constants)
   int32_t fan_off;    // offset (in doubles, even) in the program's pool:
                       // A (2^a pairs), B (2^(K-a) pairs), the constants (mask bits, 0, re, im each)
   int32_t fan_shape;  // a | kFanA (A is not all ones) | kFanB
   int32_t fan_consts; // number of constants
 };
 constexpr int32_t kFanA = 1 << 8, kFanB = 1 << 9;
-constexpr int kMaxPassFans = 64;  // constants a pass keeps in shared memory
+constexpr int kMaxPassFans = 64;  // fans with constants in a pass, which keeps them in shared memory
 
 struct TilePass {
   int32_t K;

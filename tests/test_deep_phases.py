@@ -14,7 +14,7 @@ import pytest
 from code_mojo_gb300 import butterfly as bfy
 from code_mojo_gb300 import workloads as W
 from oracle import pyoracle as O
-from tests.test_phase_fans import model, run_model  # noqa: F401 (model: a fixture)
+from tests.test_phase_fans import model, phase_mix, run_model  # noqa: F401 (model: a fixture)
 
 ROOT = Path(__file__).resolve().parent.parent
 CUDA_INC = Path("/usr/local/cuda/include")
@@ -79,3 +79,55 @@ def test_repeated_masks_match_the_oracle(model, tmp_path):  # noqa: F811
             got, _ = run_model(model, qc, re, im, K, 0, tmp_path)
             r, i = O.run(qc, re, im)
             assert np.max(np.abs(got - (r + 1j * i))) <= 4 * 400 * 2.0 ** -53  # a few roundings of 2^-53 per op
+
+
+def many_constant_fans(n, gates):
+    """A fan with a constant from outside the tile before each dense gate on
+    qubit 0 (the gates keep qubits 0 to 5 in a 6-qubit tile, and n-1 out of it)."""
+    qc = bfy.QuantumCircuit(n)
+    for k in range(gates):
+        qc.cp(n - 1, 0, 0.01 * (k + 1))
+        qc.cp(1 + k % 5, 0, 0.02 * (k + 1))
+        qc.u3(0, 0.1 * k, 0.3, 0.2)
+        qc.ry(1 + k % 5, 0.3)
+    return qc
+
+
+DEEP = {"mix": (9, 11, lambda: phase_mix(9, 2500, 5)), "mix_tiles": (12, 7, lambda: phase_mix(12, 1500, 6)),
+        "constants": (8, 6, lambda: many_constant_fans(8, 150))}
+
+
+# more fans than a pass has slots for constants: those without constants need
+# none, and phases from outside the tile stay ops once the slots are taken
+@pytest.mark.parametrize("name", list(DEEP))
+def test_more_fans_than_constants(model, name, tmp_path):  # noqa: F811
+    n, K, make = DEEP[name]
+    qc = make()
+    re, im = W.random_normal_state(n, 4)
+    got, (tiles, _, fans, phases) = run_model(model, qc, re, im, K, 0, tmp_path)
+    r, i = O.run(qc, re, im)
+    assert np.max(np.abs(got - (r + 1j * i))) <= 4 * len(qc.transformations) * 2.0 ** -53
+    if name == "constants":
+        assert fans == 64 and phases >= 150 - 64
+    else:
+        assert fans > 64 and (name != "mix" or tiles == 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+@pytest.mark.parametrize("name", list(DEEP))
+def test_more_fans_than_constants_on_the_gpu(name, dtype):
+    n, K, make = DEEP[name]
+    qc = make()
+    re, im = W.random_normal_state(n, 4)
+    ctx = bfy.ExecContext()
+    ctx.gpu_tile_qubits = K
+    st = bfy.QuantumState.from_soa(re, im, dtype)
+    bfy.execute(st, qc, ctx)
+    got = st.to_complex()
+    st.close()
+    r, i = O.run(qc, re, im)
+    exp = r + 1j * i
+    # a few roundings per op: 2^-46 in a double-float pair, 2^-24 in FP32
+    unit = 2.0 ** -46 if dtype == "c128" else 2.0 ** -24
+    assert np.linalg.norm(got - exp) <= 4 * len(qc.transformations) * unit
