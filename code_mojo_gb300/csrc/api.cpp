@@ -334,21 +334,23 @@ static void fused_pair_matrix(const bf_op& t0, const bf_op& t1, int& q_low, std:
 // the pass needs (one block costs about kBlockUnits dense gates: measured on
 // the 30-qubit complex64 layered circuit, 2.6 ms per block against 0.81 ms
 // per dense gate, beyond the 2.6 ms that moving the state costs either way).
-constexpr double kBlockUnits = 3.3;
+constexpr double kBlockUnits = 2.7;
 
-static double cuda_core_units(const std::vector<TileOp>& ops) {
+static double cuda_core_units(const std::vector<TileOp>& ops, bool fp32) {
   double u = 0;
   for (const TileOp& t : ops) {
     if (t.kind == GK_FAN) {
-      u += core_units(GK_FAN, 0);
+      u += core_units(GK_FAN, 0, fp32);
       continue;
     }
     if (t.tloc < 0) {
-      u += 0.4;  // diagonal gate on an outside target: one multiply per amplitude
+      u += core_units(GK_PHASE, 0, fp32);  // diagonal gate on an outside target: one multiply per amplitude
       continue;
     }
-    u += core_units(t.kind, t.um);
-    if (t.fan) u += core_units(GK_FAN, 0);
+    u += core_units(t.kind, t.kind == GK_UNITARY ? t.um : 0, fp32);
+    if (!t.fan) continue;
+    u += core_units(GK_FAN, 1, fp32);
+    if (t.um) u += core_units(GK_HU, 1, fp32);  // a Hadamard before the fan
   }
   return u;
 }
@@ -362,7 +364,7 @@ static double cuda_core_units(const std::vector<TileOp>& ops) {
 // The digit kernel has become faster since (a 30-qubit pass of 2.5 blocks 19.1
 // instead of 22.2 ms), but 2.1 and 1.8 plan no better: 28-qubit layered 118.9
 // and 119.0 against 118.2 ms, 27 qubits 32.9 and 32.9 against 32.8.
-constexpr double kDigitBlockUnits = 2.5;
+constexpr double kDigitBlockUnits = 2.3;
 
 // A block pass costs about this many blocks besides its blocks (loading,
 // converting and storing the tile).
@@ -418,7 +420,7 @@ static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opt
   auto flush = [&]() {
     if (run.empty()) return;
     for (auto& ps : plan_gates(n, run, K, true, tensor ? block_units : 0.0, pass_cost,
-                               tensor && format == BLOCK_DIGITS)) {
+                               tensor && format == BLOCK_DIGITS, format == BLOCK_TF32)) {
       Step s;
       if (ps.is_tile && tensor && ps.tile.K == kBlockTileQubits && ps.tile.L == kTileLowQubits) {
         size_t b0 = pg.blocks.size(), i0 = pg.images.size(), o0 = pg.offsets.size();
@@ -426,7 +428,7 @@ static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opt
         std::vector<TileOp> merged;
         int halvings = 0;
         merge_phases(ps.tile, merged, nullptr, &halvings);
-        const double cu = cuda_core_units(merged);
+        const double cu = cuda_core_units(merged, format == BLOCK_TF32);
         int max_blocks = 0;
         while (max_blocks < kMaxPassBlocks && (double)(max_blocks + 1) * block_units < cu) ++max_blocks;
         if (max_blocks > 0 &&

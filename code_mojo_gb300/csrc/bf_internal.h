@@ -436,11 +436,12 @@ struct PlanStep {
 // only a dense unitary of 4 or 5 qubits stays a pass (the complex128 digit
 // blocks run it faster than the double-float unitary kernel)
 std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int K, bool allow_single = true,
-                                 double block_units = 0, double pass_cost = 2.5, bool keep_wide_unitaries = false);
+                                 double block_units = 0, double pass_cost = 2.5, bool keep_wide_unitaries = false,
+                                 bool fp32 = false);
 
 // A tile op's cost on the CUDA cores, in units of one dense gate over the tile
 // (um: qubits of a GK_UNITARY).
-double core_units(int kind, int um);
+double core_units(int kind, int um, bool fp32);
 // The ops of a CUDA-core tile pass with their phase gates merged into phase
 // fans (see TileOp): each phase waits until a gate acts non-diagonally on one
 // of its qubits, and the phases that meet that gate's target are multiplied

@@ -641,12 +641,13 @@ static int pass_blocks(const std::vector<const GateInstr*>& remaining, uint64_t 
 // The CUDA-core tile kernel's cost of the gates a pass over inQ takes, in
 // dense-gate units (core_units of the same gates), its phases merged into
 // fans and those no gate of the pass meets left to a later one.
-static double pass_core_units(const std::vector<const GateInstr*>& remaining, uint64_t inQ, uint64_t all) {
+static double pass_core_units(const std::vector<const GateInstr*>& remaining, uint64_t inQ, uint64_t all, bool fp32) {
   uint64_t blockedX = 0, blockedAll = 0;
   double u = 0;
   // the phases that wait for a gate, one per mask (1: waiting), by qubit
   std::vector<uint64_t> by_qubit[64];
   MaskTable pending;
+  uint64_t after_h = 0;  // qubits that nothing touched since a Hadamard: a fan there takes it in
   for (const GateInstr* g : remaining) {
     const uint64_t Xg = gate_xmask(*g);
     const uint64_t Ag = gate_amask(*g);
@@ -663,43 +664,52 @@ static double pass_core_units(const std::vector<const GateInstr*>& remaining, ui
       waits = 1;
       continue;
     }
-    u += core_units(g->kind, g->um);
-    if (!Xg) continue;
-    size_t met = 0;
-    for (uint64_t b = Xg; b; b &= b - 1) {
-      std::vector<uint64_t>& l = by_qubit[__builtin_ctzll(b)];
-      for (uint64_t p : l) {
-        uint32_t& waits = pending[p];
-        met += waits;
-        waits = 0;
+    u += core_units(g->kind, g->um, fp32);
+    if (Xg) {
+      size_t met = 0;
+      for (uint64_t b = Xg; b; b &= b - 1) {
+        std::vector<uint64_t>& l = by_qubit[__builtin_ctzll(b)];
+        for (uint64_t p : l) {
+          uint32_t& waits = pending[p];
+          met += waits;
+          waits = 0;
+        }
+        l.clear();
       }
-      l.clear();
+      const bool joins = Ag == Xg && g->kind != GK_SWAP && g->kind != GK_UNITARY;
+      if (met >= (size_t)kMinFanTerms) {
+        u += core_units(GK_FAN, joins, fp32);
+        if (joins && (after_h & Xg)) u += core_units(GK_HU, 1, fp32) - core_units(GK_H, 0, fp32);
+      } else if (met) {
+        u += core_units(GK_PHASE, 0, fp32);
+      }
     }
-    if (met >= (size_t)kMinFanTerms) u += core_units(GK_FAN, 0);
-    else if (met) u += core_units(GK_PHASE, 0);
+    after_h &= ~Ag;
+    if (g->kind == GK_H) after_h |= Xg;
   }
   return u;
 }
 
-// A tile op's cost on the CUDA cores, in units of one dense gate over the
-// tile (double-float: about 134 instructions per pair, a Hadamard 58 without
-// its factor, a fan 76 on its half of the amplitudes; an m-qubit unitary does 2^m complex
-// products per amplitude against a dense gate's 2).
-double core_units(int kind, int um) {
+// Measured per op of a 12-qubit tile of 26 qubits, against a dense gate's 161
+// us (double-float) and 40 us (FP32): exchange 60 to 80 and 29 to 40, one phase
+// 61 and 22, diagonal 99 and 40, Hadamard 90 and 40 (52 and 7 within a fan's
+// op), fan 113 and 45 alone and 84 to 110 and 21 to 27 with a gate.  An m-qubit
+// unitary does 2^m complex products per amplitude against a dense gate's 2.
+double core_units(int kind, int um, bool fp32) {
   switch (kind) {
-    case GK_SWAP: return 0.5;
-    case GK_PHASE: return 0.4;
-    case GK_DIAG: return 0.6;
+    case GK_SWAP: return fp32 ? 0.8 : 0.5;
+    case GK_PHASE: return fp32 ? 0.55 : 0.4;
+    case GK_DIAG: return fp32 ? 1.0 : 0.6;
     case GK_H:
-    case GK_HU: return 0.45;
-    case GK_FAN: return 0.6;
+    case GK_HU: return um ? (fp32 ? 0.17 : 0.32) : (fp32 ? 1.0 : 0.45);
+    case GK_FAN: return um || !fp32 ? 0.6 : 1.1;
     case GK_UNITARY: return (double)(1 << (um - 1));
     default: return 1.0;
   }
 }
 
 std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int K, bool allow_single,
-                                 double block_units, double pass_cost, bool keep_wide_unitaries) {
+                                 double block_units, double pass_cost, bool keep_wide_unitaries, bool fp32) {
   std::vector<PlanStep> steps;
   if (gates.empty()) return steps;
   K = std::max(1, std::min(K, std::min(n, kMaxTileQubits)));
@@ -784,8 +794,8 @@ std::vector<PlanStep> plan_gates(int n, const std::vector<GateInstr>& gates, int
         // costs block_units dense gates).
         auto block_rate = [&](uint64_t c) { return work(c) / (pass_cost + pass_blocks(remaining, c, all)); };
         const uint64_t set = search(start, block_rate);
-        const double core = pass_core_units(remaining, set, all);
-        const double core_rate = work(by_work) / (pass_cost + pass_core_units(remaining, by_work, all) / block_units);
+        const double core = pass_core_units(remaining, set, all, fp32);
+        const double core_rate = work(by_work) / (pass_cost + pass_core_units(remaining, by_work, all, fp32) / block_units);
         if ((double)pass_blocks(remaining, set, all) * block_units < core && block_rate(set) >= core_rate) {
           inQ = set;
           blocks_chosen = true;
