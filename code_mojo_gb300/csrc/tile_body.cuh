@@ -137,6 +137,9 @@ __device__ __forceinline__ void tile_pairs_fan(typename P::Smem* amp, int TS, in
 // local bit 0, or for a target on bit 0 one pair).  The passes of a 27-qubit
 // value encoding take 4.74 against 6.66 ms, of six layers of U3 and CX at 24
 // qubits 2.17 against 2.33.
+// The loops stay rolled: unrolled by two, the kinds of a mixed circuit no longer
+// fit the instruction cache (500 gates of every kind at 24 qubits 5.20 ms, 4.66
+// like this, 4.80 one amplitude at a time; a batch of 128 circuits 702 and 665 us).
 struct Pair32 {
   PolF32::R a, b;  // local bit 0 = 0, 1
 };
@@ -180,7 +183,7 @@ __device__ __forceinline__ void tile_words(float2* amp, int TS, int tloc, uint32
   using P = PolF32;
   float4* amp4 = reinterpret_cast<float4*>(amp);
   if (tloc == 0) {
-#pragma unroll 2
+#pragma unroll 1
     for (int k = threadIdx.x; k < (TS >> 1); k += kTileThreads) {
       if (kCtl && ((uint32_t)(2 * k) & cml) != cml) continue;
       Pair32 p = pair32(amp4[k]);
@@ -200,7 +203,7 @@ __device__ __forceinline__ void tile_words(float2* amp, int TS, int tloc, uint32
   const uint32_t low = (1u << (tloc - 1)) - 1u, tb = 1u << (tloc - 1);
   const uint32_t need = cml >> 1;
   const bool odd_only = kCtl && (cml & 1u);
-#pragma unroll 2
+#pragma unroll 1
   for (uint32_t q = threadIdx.x; q < (uint32_t)(TS >> 2); q += kTileThreads) {
     const uint32_t w0 = ((q & ~low) << 1) | (q & low), w1 = w0 | tb;
     if (kCtl && (w0 & need) != need) continue;
