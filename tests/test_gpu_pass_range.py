@@ -124,3 +124,37 @@ def test_complex64_value_encoding_stays_near_fp32(n):
         r, i = O.run(qc, *O.basis(n))
         d = got - (r + 1j * i)
         assert np.max(np.abs(d)) <= bound and np.linalg.norm(d) <= bound
+
+
+@pytest.mark.parametrize("dtype", ["c128", "c64"])
+@pytest.mark.parametrize("times", [2, 24])
+def test_factors_over_the_exponent_range(dtype, times):
+    """H an even number of times on one qubit, 1 and 12 powers of two at the
+    store, on amplitudes from below the smallest values a pair keeps whole up
+    to where a pass scales its tiles before the gates (2^100) and beyond.
+
+    Each H rounds by a few units of the larger amplitude of the pair; below,
+    an absolute 2^-100 (what a pair drops, with the tile scaled by 2^-12)."""
+    n = 14
+    rng = np.random.Generator(np.random.PCG64(times))
+    e = rng.integers(-140, 100, 1 << n)
+    e[1 << 9:3 << 9] = rng.integers(-40, 125, 2 << 9)   # tiles with large amplitudes beside tiles without
+    e[5 << 9:6 << 9] = rng.integers(98, 102, 1 << 9)
+    x = np.ldexp(rng.uniform(1, 2, (2, 1 << n)) * rng.choice([-1.0, 1.0], (2, 1 << n)), e)
+    if dtype == "c64":
+        x = x.astype(np.float32).astype(np.float64)
+    qc = bfy.QuantumCircuit(n)
+    for _ in range(times):
+        qc.h(3)
+    ctx = bfy.ExecContext()
+    ctx.gpu_tile_qubits = 9
+    ctx.gpu_tensor_blocks = False
+    ctx.gpu_renormalize = False
+    st = bfy.QuantumState.from_soa(x[0], x[1], dtype)
+    bfy.execute(st, qc, ctx)
+    got = np.array(st.download())
+    st.close()
+    pair = np.abs(x).max(0).reshape(-1, 2, 8)           # qubit 3
+    top = np.broadcast_to(pair.max(1, keepdims=True), pair.shape).reshape(-1)
+    unit = 2.0 ** -24 if dtype == "c64" else 2.0 ** -45
+    assert np.all(np.abs(got - x).max(0) <= 4 * times * unit * top + 2.0 ** -100)
