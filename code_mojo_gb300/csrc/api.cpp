@@ -331,9 +331,11 @@ static void fused_pair_matrix(const bf_op& t0, const bf_op& t1, int& q_low, std:
 
 // Tensor cores or CUDA cores for one 12-qubit pass: the CUDA-core tile
 // kernel's work in units of one dense gate over the tile, against the blocks
-// the pass needs (one block costs about kBlockUnits dense gates: measured on
-// the 30-qubit complex64 layered circuit, 2.6 ms per block against 0.81 ms
-// per dense gate, beyond the 2.6 ms that moving the state costs either way).
+// the pass needs.  A complex64 block takes 114 us at 26 qubits and a dense gate
+// of an FP32 tile 40 us (9.1 and 3.2 at 22, 2.9 and 1.15 at 20 qubits).  With
+// 2.9, 2.7, 2.6 and 2.3: 2500 mixed gates of 16 qubits 1320, 1224, 1234, 1192
+// us; 300 of 26 qubits 8.12, 7.78, 7.79, 8.13 ms; 5 ZZ layers of 20 qubits 207,
+// 177, 179, 179 us; the 24-qubit QFT 643, 639, 684, 683 us.
 constexpr double kBlockUnits = 2.7;
 
 static double cuda_core_units(const std::vector<TileOp>& ops, bool fp32) {
@@ -355,15 +357,11 @@ static double cuda_core_units(const std::vector<TileOp>& ops, bool fp32) {
   return u;
 }
 
-// complex128 digit blocks against the double-float tile kernel: one block
-// costs about this many double-float dense gates (on the 30-qubit layered
-// circuit a digit pass costs about 8 ms plus 5.8 ms per block, a dense gate
-// in a double-float tile pass about 2.4 ms).  Measured against 5.0: the
-// 30-qubit circuit 1144 against 1152 ms, value encoding at 22, 24 and 25
-// (fused pairs) qubits 1.95 / 5.25 / 10.8 against 2.47 / 7.00 / 13.6 ms.
-// The digit kernel has become faster since (a 30-qubit pass of 2.5 blocks 19.1
-// instead of 22.2 ms), but 2.1 and 1.8 plan no better: 28-qubit layered 118.9
-// and 119.0 against 118.2 ms, 27 qubits 32.9 and 32.9 against 32.8.
+// complex128 digit blocks against the double-float tile kernel: a block takes
+// 304 us at 26 qubits, a dense gate 161 us (19.5 and 10.9 at 22 qubits).  With
+// 2.5, 2.3, 2.1 and 1.9: 2500 mixed gates of 16 qubits 2.67, 2.35, 2.23, 2.16
+// ms; 500 of 24 qubits 9.29, 8.67, 8.55, 8.55 ms; 24-qubit order finding 1.706,
+// 1.706, 1.786, 1.787 ms; layered circuits the same plans.
 constexpr double kDigitBlockUnits = 2.3;
 
 // A block pass costs about this many blocks besides its blocks (loading,

@@ -45,9 +45,9 @@ constexpr int kMargPer = (1 << kMargTileBits) / kMeasThreads;     // tile positi
 // Bound by HBM: the state is read once in 32 KiB runs (8 independent 16-byte
 // loads per thread in flight).  One CTA per outcome, which this replaces, read
 // 2^20 outcomes of 16 amplitudes as 2^20 CTAs and finished them on the host.
-// A 20-qubit register of 24 (complex128): 5.33 ms then, 0.70 ms now, most of
-// it the 8 MiB result's copy; 16 of 28 (complex128): 2.97 against 0.87 ms,
-// 0.72 of the copy bandwidth; 16 of 29 (complex64): 5.22 against 0.87 ms.
+// A 20-qubit register of 24 (complex128): 5.26 ms then, 0.64 ms now, most of
+// it the 8 MiB result's copy; 16 of 28 (complex128): 2.64 against 0.75 ms,
+// 0.84 of the copy bandwidth; 16 of 29 (complex64): 5.19 against 0.70 ms.
 enum { kMargRun, kMargSpread, kMargPart };  // a contiguous tile, a whole one, less than one
 struct MargArgs {
   int32_t tile_bits;       // T
@@ -298,7 +298,10 @@ const double* marginal_probs(State& st, const int32_t* q, const int8_t* values, 
   for (int j = 0; j < kMargPer; ++j) a.row[j] = deposit_mask((uint64_t)j * kMeasThreads, a.tile_mask);
   a.steps = 1ull << __builtin_popcountll(a.sum_high);
   a.outcomes = 1ull << nfree;
-  // One wave of CTAs; a chunk is whole walk steps, at least one per 512
+  // One wave of CTAs for one setting of the free high qubits (28 qubits, none
+  // free, complex128: 742 against 800 us with 8 CTAs per SM), more where only
+  // halves and quarters of a wave could be had (8 high ones free: 703 against
+  // 883, complex64 365 against 351); a chunk is whole walk steps, at least one per 512
   // outcomes it writes (so that the sums stay a fraction of what is read), and
   // the chunks' sums stay within 32 MiB
   uint64_t chunks = std::max<uint64_t>(1, ((uint64_t)st.num_sms * (nfh ? 8 : kMargCtas)) >> nfh);

@@ -70,10 +70,10 @@ __device__ __forceinline__ void tile_gate(int kind, typename P::Smem* amp, int T
 // of it behind a barrier.  The n(n-1)/2 phases of a Fourier transform become
 // at most one fan per Hadamard, multiplied into the pair the Hadamard has in
 // registers anyway: one or two complex products per pair whatever the number
-// of phases.  At 24 qubits, complex128, the value encoding (24 P, 276 CP, 48
-// H) took 4.13 ms as 46 digit blocks in 4 passes and takes 1.64 ms in 3 tile
-// passes with fans; at 27 qubits, complex64, 17.3 against 4.3 ms; the 20-qubit
-// QFT's passes, complex128, 0.30 against 0.11 ms.
+// of phases.  At 24 qubits, complex128, executing the value encoding (24 P, 276
+// CP, 48 H) took 5.39 ms as 46 digit blocks in 4 passes and takes 1.68 ms in 3
+// tile passes with fans; at 27 qubits, complex64, 18.2 against 5.1 ms; the
+// 20-qubit QFT, complex128, 0.40 against 0.12 ms.
 //
 // A phase fan as the CTA holds it: tables in shared memory (the constant
 // folded into one of them), or with neither table the constant alone.
