@@ -625,7 +625,10 @@ void batch_download(Batch& b, int c, double* re, double* im) {
   };
   if (N * eb > (b.dtype == BF_C128 ? kBatchDirect128 : kBatchDirect64)) {
     BatchStage stage(b);
-    if (stage->reserve(N)) {
+    // room for the batch's largest circuit at once: growing from size to size
+    // allocates pinned memory several times in a first reading
+    const uint64_t largest = 1ull << *std::max_element(b.nq.begin(), b.nq.end());
+    if (stage->reserve(largest)) {
       stage->download(N, re, im, b.stream, convert);
       return;
     }
