@@ -120,6 +120,9 @@ __device__ __forceinline__ void load_word(float4& v, const void* p) {
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                : "l"(p));
 }
+__device__ __forceinline__ void load_word(float2& v, const void* p) {
+  asm volatile("ld.global.cs.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+}
 __device__ __forceinline__ dfl word_norm2_df(double2 w) { return amp_norm2_df<double2>(w); }
 __device__ __forceinline__ dfl word_norm2_df(float4 w) {
   return df_add(amp_norm2_df<float2>(make_float2(w.x, w.y)), amp_norm2_df<float2>(make_float2(w.z, w.w)));
@@ -207,7 +210,10 @@ double reduce_norm2(State& st) {
 // sum conj(a_i) b_i over two states of the same size and either dtype, in
 // double-float per thread; partials (re.hi, re.lo, im.hi, im.lo) per block
 // summed on the host in FP64.  Used for the fidelity of a complex64 result
-// against a complex128 one.
+// against a complex128 one.  Bound by HBM: four loads of either state in flight
+// per thread, which the compiler no longer kept once the conversions between
+// them became shorter (28 qubits, complex128, 1395 -> 1580 us; 1433 like this,
+// complex64 718 -> 670, one of each 1151 -> 990).
 template <class T>
 __device__ __forceinline__ void amp_df2(T a, dfl& re, dfl& im);
 template <>
@@ -227,13 +233,27 @@ __global__ void __launch_bounds__(256) k_inner(const TA* __restrict__ a, const T
   __shared__ dfl wr[8], wi[8];
   dfl sr{0.f, 0.f}, si{0.f, 0.f};
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += step) {
+  auto add = [&](TA x, TB y) {
     dfl ar, ai, br, bi;
-    amp_df2<TA>(a[i], ar, ai);
-    amp_df2<TB>(b[i], br, bi);
+    amp_df2<TA>(x, ar, ai);
+    amp_df2<TB>(y, br, bi);
     sr = df_add(sr, df_dot2(ar, br, ai, bi));           // re(conj(a) b) = ar br + ai bi
     si = df_add(si, df_dot2(ar, bi, df_neg(ai), br));   // im(conj(a) b) = ar bi - ai br
+  };
+  constexpr int kU = 4;
+  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + (kU - 1) * step < N; i += kU * step) {
+    TA va[kU];
+    TB vb[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      load_word(va[u], a + i + u * step);
+      load_word(vb[u], b + i + u * step);
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) add(va[u], vb[u]);
   }
+  for (; i < N; i += step) add(a[i], b[i]);
   for (int off = 16; off > 0; off >>= 1) {
     sr = df_shfl_add(sr, off);
     si = df_shfl_add(si, off);
@@ -262,7 +282,11 @@ __global__ void __launch_bounds__(256) k_inner(const TA* __restrict__ a, const T
 
 void inner_product(State& a, State& b, double* re, double* im) {
   if (a.n != b.n) fail(BF_EINVAL, "inner product of states with %d and %d qubits", a.n, b.n);
-  unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.N + 255) / 256, (uint64_t)a.num_sms * 8));
+  // twice the CTAs for large states, where the last ones' tail counts for more
+  // than the partials' readback (28 qubits, complex128, 1433 against 1493 us; at
+  // 23 qubits 71 against 69.5)
+  const uint64_t per_sm = a.n >= 25 ? 16 : 8;
+  unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.N + 255) / 256, (uint64_t)a.num_sms * per_sm));
   ensure_partials(a, 2 * (size_t)blocks, 2 * (size_t)blocks);
   // b's pending work must finish before a's stream reads it
   cudaEvent_t ev;
