@@ -426,9 +426,16 @@ static void build_steps(int n, const bf_op* ops, int64_t nops, const bf_exec_opt
         std::vector<TileOp> merged;
         int halvings = 0;
         merge_phases(ps.tile, merged, nullptr, &halvings);
-        const double cu = cuda_core_units(merged, format == BLOCK_TF32);
+        // (a digit pass has to save half a dense gate: the scale before a circuit's
+        // first one is a sweep of its own; a chain of CX on 17 qubits took 64 us
+        // with one digit block that was to save a fifth of a gate, 54 without)
+        const double cu = cuda_core_units(merged, format == BLOCK_TF32) - (format == BLOCK_DIGITS ? 0.5 : 0.0);
+        // a pass of diagonal ops alone keeps its tile form (a layer of phases on
+        // 26 qubits, complex64, 1193 us, as five blocks 1383)
+        const bool mixes = std::any_of(ps.tile.ops.begin(), ps.tile.ops.end(),
+                                       [](const TileOp& t) { return t.kind != GK_PHASE && t.kind != GK_DIAG; });
         int max_blocks = 0;
-        while (max_blocks < kMaxPassBlocks && (double)(max_blocks + 1) * block_units < cu) ++max_blocks;
+        while (mixes && max_blocks < kMaxPassBlocks && (double)(max_blocks + 1) * block_units < cu) ++max_blocks;
         if (max_blocks > 0 &&
             plan_blocks(ps.tile, pg.blocks, pg.images, pg.offsets, format, max_blocks, pg.umats.data()) &&
             (double)(pg.blocks.size() - b0) * block_units < cu) {
