@@ -158,3 +158,32 @@ def test_factors_over_the_exponent_range(dtype, times):
     top = np.broadcast_to(pair.max(1, keepdims=True), pair.shape).reshape(-1)
     unit = 2.0 ** -24 if dtype == "c64" else 2.0 ** -45
     assert np.all(np.abs(got - x).max(0) <= 4 * times * unit * top + 2.0 ** -100)
+
+
+@pytest.mark.parametrize("n,K", [(14, 5), (13, 4)])
+def test_complex64_constants_round_once(n, K):
+    """A phase on every set of the qubits outside the tile and one inside, then
+    a Hadamard there: the constant of the fan is a product of up to 2^(n-K)
+    factors and has to come out as one rounded number.
+
+    Bound by pairs, in units of 2^-24 of a pair's norm: 1 for the constant,
+    sqrt(5) for a complex product, 3 for the Hadamard (sum, factor, product);
+    a constant whose products are rounded one by one is off by about 14."""
+    rng = np.random.Generator(np.random.PCG64(n))
+    qc = bfy.QuantumCircuit(n)
+    for m in range(1, 1 << (n - K)):
+        qc.mcp([K + j for j in range(n - K) if m >> j & 1], 2, float(rng.uniform(-3, 3)))
+    qc.h(2)
+    re, im = (x.astype(np.float32).astype(np.float64) for x in W.random_normal_state(n, 5))
+    ctx = bfy.ExecContext()
+    ctx.gpu_tile_qubits = K
+    ctx.gpu_tensor_blocks = False
+    ctx.gpu_renormalize = False
+    st = bfy.QuantumState.from_soa(re, im, "c64")
+    bfy.execute(st, qc, ctx)
+    gr, gi = st.download()
+    st.close()
+    r, i = O.run(qc, re, im)
+    pairs = lambda x: np.sqrt((np.abs(x).reshape(-1, 2, 4) ** 2).sum(1))
+    err = pairs((gr - r) + 1j * (gi - i)) / pairs(r + 1j * i)
+    assert np.max(err) <= (1 + np.sqrt(5) + 3) * 2.0 ** -24
